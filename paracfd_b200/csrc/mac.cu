@@ -16,8 +16,10 @@
 //   diffusion explicit 7-point face Laplacian with nu + mean nut of the two cells across the
 //             face; band faces use only their open links and molecular nu (:709-713)
 // Samples that leave a brick take the same-level neighbour across one face, else the finest brick
-// that contains the lattice node (one-sided linear extension across 2:1 transitions).  One launch
-// covers all brick slots of all levels; covered bricks are skipped (their output faces are 0, as
+// that contains the lattice node (one-sided linear extension across 2:1 transitions).  That value
+// depends on the node alone, so each field is first copied into per-brick lattices with one ghost
+// node all round (extend): every sample then reads its eight nodes from one brick's lattice.  One
+// launch covers all brick slots of all levels; covered bricks are skipped (their output faces are 0, as
 // the reference's scratch commit leaves them).  The link bytes are the caller's preprocessing
 // (the fabric band and its open directions come from the caller's surface BVH).
 #include "locator.h"
@@ -37,6 +39,7 @@ namespace pcfd
             const uint32_t* flags;      // [B] brick flags by slot
             const int* slot_level;      // [B]
             int bs;
+            const float* ext;           // the sampled field's extended lattices (ext_index), one ghost node all round
         };
         struct Faces
         {
@@ -54,13 +57,28 @@ namespace pcfd
         }
         __device__ inline bool covered(const MacView& m, int64_t slot) { return (m.flags[slot] & PCFD_BRICK_COVERED) != 0; }
 
-        // face value with indices clamped to the component's lattice of the brick
-        __device__ inline float clamped(const Faces& f, int bs, int c, int64_t slot, int i, int j, int k)
+        // face index / value with indices clamped to the component's lattice of the brick
+        __device__ inline int64_t clamped_face(int bs, int c, int64_t slot, int i, int j, int k)
         {
             i = max(0, min(c == 0 ? bs : bs - 1, i));
             j = max(0, min(c == 1 ? bs : bs - 1, j));
             k = max(0, min(c == 2 ? bs : bs - 1, k));
-            return f.c[c][axis_face(bs, c, slot, i, j, k)];
+            return axis_face(bs, c, slot, i, j, k);
+        }
+        __device__ inline float clamped(const Faces& f, int bs, int c, int64_t slot, int i, int j, int k)
+        {
+            return f.c[c][clamped_face(bs, c, slot, i, j, k)];
+        }
+        // Extended lattice of component c of brick `slot`: its nodes -1 .. n per axis, [slot][c][k][j][i].
+        __host__ __device__ inline int ext_size(int bs) { return (bs + 3) * (bs + 2) * (bs + 2); }
+        __device__ inline bool in_extended(int c, int bs, int i, int j, int k)
+        {
+            return i >= -1 && j >= -1 && k >= -1 && i <= (c == 0 ? bs + 1 : bs) && j <= (c == 1 ? bs + 1 : bs) && k <= (c == 2 ? bs + 1 : bs);
+        }
+        __device__ inline int64_t ext_index(int c, int bs, int64_t slot, int i, int j, int k)
+        {
+            const int nx = c == 0 ? bs + 3 : bs + 2, ny = c == 1 ? bs + 3 : bs + 2;
+            return (slot * 3 + c) * ext_size(bs) + ((k + 1) * ny + j + 1) * nx + i + 1;
         }
         // one-sided linear extension past the lattice ends (weights 2, -1 per axis)
         __device__ float extended(const Faces& f, int bs, int c, int64_t slot, int i, int j, int k)
@@ -134,12 +152,15 @@ namespace pcfd
             else if (face == 3) j -= bs; else if (face == 4) k += bs; else k -= bs;
         }
 
-        // value of lattice node (i,j,k) of component c of brick `slot` (level `level`), which may
-        // lie outside the brick
-        __device__ __noinline__ float node_value(const MacView& m, const Faces& f, int level, int64_t slot, int c, int i, int j, int k)
+        // Where the value of lattice node (i,j,k) of component c of brick `slot` (level `level`) comes
+        // from, which may lie outside the brick: the index of one face of the component, or -1 when it
+        // is interpolated on another level's brick `at` (at the node's position nx, ny, nz).  It
+        // depends on the grid only.
+        __device__ inline int64_t node_source(const MacView& m, int level, int64_t slot, int c, int i, int j, int k, int& at, int& at_level,
+                                              float& nx, float& ny, float& nz)
         {
             const int bs = m.bs;
-            if (valid_face(c, bs, i, j, k)) return clamped(f, bs, c, slot, i, j, k);
+            if (valid_face(c, bs, i, j, k)) return axis_face(bs, c, slot, i, j, k);
             const int face = outside_face(c == 0 ? bs + 1 : bs, c == 1 ? bs + 1 : bs, c == 2 ? bs + 1 : bs, i, j, k);
             if (face >= 0)
             {
@@ -147,25 +168,37 @@ namespace pcfd
                 if (nb >= 0 && !covered(m, nb))
                 {
                     shift_into(face, bs, i, j, k);
-                    return clamped(f, bs, c, nb, i, j, k);
+                    return clamped_face(bs, c, nb, i, j, k);
                 }
             }
             const float4 rec = record_of(m, level, slot);
-            float nx, ny, nz;
             face_point(rec, c, i, j, k, nx, ny, nz);
             const float* lo = m.loc.lo;
             const float* hi = m.loc.hi;
-            if (nx < lo[0] || ny < lo[1] || nz < lo[2] || nx > hi[0] || ny > hi[1] || nz > hi[2]) return clamped(f, bs, c, slot, i, j, k);
+            if (nx < lo[0] || ny < lo[1] || nz < lo[2] || nx > hi[0] || ny > hi[1] || nz > hi[2]) return clamped_face(bs, c, slot, i, j, k);
             const float eps = 1e-5f * rec.w;
             const float px = fminf(hi[0] - eps, fmaxf(lo[0] + eps, nx)), py = fminf(hi[1] - eps, fmaxf(lo[1] + eps, ny)),
                         pz = fminf(hi[2] - eps, fmaxf(lo[2] + eps, nz));
-            int at_level;
-            const int at = locate(m, px, py, pz, at_level);
-            if (at < 0) return clamped(f, bs, c, slot, i, j, k);
+            at = locate(m, px, py, pz, at_level);
+            if (at < 0) return clamped_face(bs, c, slot, i, j, k);
+            if (at_level != level) return -1;
             const float4 r = record_of(m, at_level, at);
-            if (at_level != level) return sample_extended(f, bs, r, c, at, nx, ny, nz);
-            return clamped(f, bs, c, at, nearest_index(nx, r.x, r.w, c == 0 ? 0.0f : 0.5f), nearest_index(ny, r.y, r.w, c == 1 ? 0.0f : 0.5f),
-                           nearest_index(nz, r.z, r.w, c == 2 ? 0.0f : 0.5f));
+            return clamped_face(bs, c, at, nearest_index(nx, r.x, r.w, c == 0 ? 0.0f : 0.5f), nearest_index(ny, r.y, r.w, c == 1 ? 0.0f : 0.5f),
+                                nearest_index(nz, r.z, r.w, c == 2 ? 0.0f : 0.5f));
+        }
+        __device__ __noinline__ float node_value(const MacView& m, const Faces& f, int level, int64_t slot, int c, int i, int j, int k)
+        {
+            int at = -1, at_level = -1;
+            float nx, ny, nz;
+            const int64_t source = node_source(m, level, slot, c, i, j, k, at, at_level, nx, ny, nz);
+            if (source >= 0) return f.c[c][source];
+            return sample_extended(f, m.bs, record_of(m, at_level, at), c, at, nx, ny, nz);
+        }
+        // cell i0 (fraction x) moved to the last cell [-1, top] when it is past it by rounding only
+        __device__ inline void settle(float& x, int& i0, int top)
+        {
+            if (i0 == -2 && x > 0.999f) { i0 = -1; x -= 1.0f; }
+            else if (i0 == top + 1 && x < 0.001f) { i0 = top; x += 1.0f; }
         }
         // trilinear sample of component c at p from brick `slot`'s lattice, with the range of the
         // eight node values
@@ -176,24 +209,38 @@ namespace pcfd
             float x = (px - rec.x) / rec.w - (c == 0 ? 0.0f : 0.5f);
             float y = (py - rec.y) / rec.w - (c == 1 ? 0.0f : 0.5f);
             float z = (pz - rec.z) / rec.w - (c == 2 ? 0.0f : 0.5f);
-            const int i0 = int(floorf(x)), j0 = int(floorf(y)), k0 = int(floorf(z));
+            int i0 = int(floorf(x)), j0 = int(floorf(y)), k0 = int(floorf(z));
             x -= i0;
             y -= j0;
             z -= k0;
-            float result = 0, mn = 0, mx = 0;
-            bool first = true;
-            for (int dz = 0; dz < 2; ++dz)
-                for (int dy = 0; dy < 2; ++dy)
-                    for (int dx = 0; dx < 2; ++dx)
-                    {
-                        const int ni = i0 + dx, nj = j0 + dy, nk = k0 + dz;
-                        const float wx = dx ? x : 1.0f - x, wy = dy ? y : 1.0f - y, wz = dz ? z : 1.0f - z;
-                        const float value = valid_face(c, bs, ni, nj, nk) ? clamped(f, bs, c, slot, ni, nj, nk)
-                                                                          : node_value(m, f, level, slot, c, ni, nj, nk);
-                        result += wx * wy * wz * value;
-                        if (first) { mn = mx = value; first = false; }
-                        else { mn = fminf(mn, value); mx = fmaxf(mx, value); }
-                    }
+            // a sample that rounding put a hair outside the extended lattice's end nodes extends the
+            // last cell by that hair instead of reaching for one more node
+            settle(x, i0, c == 0 ? bs : bs - 1);
+            settle(y, j0, c == 1 ? bs : bs - 1);
+            settle(z, k0, c == 2 ? bs : bs - 1);
+            float v[8];
+            if (in_extended(c, bs, i0, j0, k0) && in_extended(c, bs, i0 + 1, j0 + 1, k0 + 1))
+            {
+                const float* e = m.ext + ext_index(c, bs, slot, i0, j0, k0);
+                const int nx = c == 0 ? bs + 3 : bs + 2, nxy = nx * (c == 1 ? bs + 3 : bs + 2);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = e[(q & 1) + (q >> 1 & 1) * nx + (q >> 2) * nxy];
+            }
+            else
+            {
+                // past the extended lattice (not reached by the characteristics of a CFL-limited step)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = node_value(m, f, level, slot, c, i0 + (q & 1), j0 + (q >> 1 & 1), k0 + (q >> 2));
+            }
+            float result = 0, mn = v[0], mx = v[0];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+            {
+                const float wx = q & 1 ? x : 1.0f - x, wy = q & 2 ? y : 1.0f - y, wz = q & 4 ? z : 1.0f - z;
+                result += wx * wy * wz * v[q];
+                mn = fminf(mn, v[q]);
+                mx = fmaxf(mx, v[q]);
+            }
             if (lower) *lower = mn;
             if (upper) *upper = mx;
             return result;
@@ -209,34 +256,52 @@ namespace pcfd
             y = fminf(m.loc.hi[1] - 1e-5f, fmaxf(m.loc.lo[1] + 1e-5f, y));
             z = fminf(m.loc.hi[2] - 1e-5f, fmaxf(m.loc.lo[2] + 1e-5f, z));
         }
-        // sample on the finest brick owning p (clamped into the domain); `fallback` when none does
-        __device__ float sample_finest(const MacView& m, const Faces& f, int c, float x, float y, float z, float fallback, float* lower,
-                                       float* upper)
+        // locate() for points near brick `home` (non-covered, level `level`): no finer brick lies in
+        // a non-covered one and the level widths are exact halves, so a point whose brick coordinates
+        // are the home brick's is in it and needs no search from the finest level down.
+        struct Home
         {
-            clamp_point(m, x, y, z);
+            int64_t slot;
             int level;
-            const int at = locate(m, x, y, z, level);
-            if (at < 0)
-            {
-                if (lower) *lower = fallback;
-                if (upper) *upper = fallback;
-                return fallback;
-            }
-            return sample_bounded(m, f, level, at, record_of(m, level, at), c, x, y, z, lower, upper);
-        }
-        // two-stage characteristic from p over dt (negative dt traces forward)
-        __device__ void trace(const MacView& m, const Faces& f, int level, int64_t slot, const float4& rec, float& x, float& y, float& z,
-                              float dt)
+            float width, bx, by, bz;    // brick width, brick coordinates as locate() rounds them
+        };
+        __device__ inline Home home_of(const MacView& m, int level, int64_t slot, const float4& rec)
         {
-            const float ux = sample(m, f, level, slot, rec, 0, x, y, z), uy = sample(m, f, level, slot, rec, 1, x, y, z),
-                        uz = sample(m, f, level, slot, rec, 2, x, y, z);
-            float mx = x - float(0.5f * dt * ux), my = y - float(0.5f * dt * uy), mz = z - float(0.5f * dt * uz);
+            Home h{slot, level, float(m.bs) * m.loc.levels[level].h, 0.0f, 0.0f, 0.0f};
+            const float half = 0.5f * h.width;
+            h.bx = floorf((rec.x + half - m.loc.lo[0]) / h.width);
+            h.by = floorf((rec.y + half - m.loc.lo[1]) / h.width);
+            h.bz = floorf((rec.z + half - m.loc.lo[2]) / h.width);
+            return h;
+        }
+        __device__ inline int locate_near(const MacView& m, const Home& h, float x, float y, float z, int& level)
+        {
+            const bool inside = x >= m.loc.lo[0] && y >= m.loc.lo[1] && z >= m.loc.lo[2] && x < m.loc.hi[0] && y < m.loc.hi[1] && z < m.loc.hi[2];
+            if (inside && floorf((x - m.loc.lo[0]) / h.width) == h.bx && floorf((y - m.loc.lo[1]) / h.width) == h.by &&
+                floorf((z - m.loc.lo[2]) / h.width) == h.bz)
+            {
+                level = h.level;
+                return int(h.slot);
+            }
+            return locate(m, x, y, z, level);
+        }
+        // two-stage characteristic from p over dt (negative dt traces forward); u: the velocity at p
+        __device__ void trace(const MacView& m, const Faces& f, const Home& home, const float u[3], float& x, float& y, float& z, float dt)
+        {
+            float mx = x - float(0.5f * dt * u[0]), my = y - float(0.5f * dt * u[1]), mz = z - float(0.5f * dt * u[2]);
             clamp_point(m, mx, my, mz);
-            const float vx = sample_finest(m, f, 0, mx, my, mz, ux, nullptr, nullptr), vy = sample_finest(m, f, 1, mx, my, mz, uy, nullptr, nullptr),
-                        vz = sample_finest(m, f, 2, mx, my, mz, uz, nullptr, nullptr);
-            x = x - float(dt * vx);
-            y = y - float(dt * vy);
-            z = z - float(dt * vz);
+            int level;
+            const int at = locate_near(m, home, mx, my, mz, level);
+            float v[3] = {u[0], u[1], u[2]};
+            if (at >= 0)
+            {
+                const float4 rec = record_of(m, level, at);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) v[c] = sample(m, f, level, at, rec, c, mx, my, mz);
+            }
+            x = x - float(dt * v[0]);
+            y = y - float(dt * v[1]);
+            z = z - float(dt * v[2]);
             clamp_point(m, x, y, z);
         }
         __device__ inline void decode(int64_t q, int bs, int& c, int64_t& slot, int& i, int& j, int& k)
@@ -322,7 +387,73 @@ namespace pcfd
             float* c[3];
         };
 
-        __global__ void mac_forward_kernel(MacView m, Faces f, Links links, int64_t total, float dt, Out out)
+        // Source of every node of every extended lattice: the index of a face of the component, -1 for
+        // the nodes interpolated on another level (they are counted, and listed when `slow` is
+        // given), -2 in covered bricks (never sampled).
+        __global__ void mac_source_kernel(MacView m, int64_t total, int* source, int* slow, int* count)
+        {
+            const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+            if (q >= total) return;
+            const int bs = m.bs, per = ext_size(bs);
+            const int64_t slot = q / (3 * per);
+            const int c = int(q / per % 3);
+            int local = int(q % per);
+            const int nx = c == 0 ? bs + 3 : bs + 2, ny = c == 1 ? bs + 3 : bs + 2;
+            const int i = local % nx - 1;
+            local /= nx;
+            const int j = local % ny - 1, k = local / ny - 1;
+            if (covered(m, slot)) { source[q] = -2; return; }
+            int at = -1, at_level = -1;
+            float x, y, z;
+            const int64_t from = node_source(m, m.slot_level[slot], slot, c, i, j, k, at, at_level, x, y, z);
+            source[q] = int(from);
+            if (from < 0)
+            {
+                const int n = atomicAdd(count, 1);
+                if (slow) slow[n] = int(q);
+            }
+        }
+        // Extended lattices of a field: copies, then the listed nodes interpolated on another level.
+        // The copy is bound by memory (4 B source, 4 B value, 4 B store per node; 3 x 1100 nodes per
+        // 8^3 brick); the interpolation's 64 clamped reads per node run in a launch of their own, so
+        // no copying warp waits for them.
+        __global__ void mac_extend_kernel(Faces f, int per, int64_t total, const int* __restrict__ source, float* __restrict__ ext)
+        {
+            const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+            if (q >= total) return;
+            const int from = source[q];
+            if (from >= 0) ext[q] = f.c[int(q / per % 3)][from];
+        }
+        __global__ void mac_extend_slow_kernel(MacView m, Faces f, int count, const int* __restrict__ slow, float* __restrict__ ext)
+        {
+            const int n = blockIdx.x * blockDim.x + threadIdx.x;
+            if (n >= count) return;
+            const int q = slow[n];
+            const int bs = m.bs, per = ext_size(bs);
+            const int64_t slot = q / (3 * per);
+            const int c = q / per % 3;
+            int local = q % per;
+            const int nx = c == 0 ? bs + 3 : bs + 2, ny = c == 1 ? bs + 3 : bs + 2;
+            const int i = local % nx - 1;
+            local /= nx;
+            ext[q] = node_value(m, f, m.slot_level[slot], slot, c, i, local % ny - 1, local / ny - 1);
+        }
+
+        // What the correction of a face needs from the forward pass: the forward foot, the range of the
+        // backward foot's samples and the brick that owns the forward foot (-1: no correction).
+        struct Feet
+        {
+            float4* foot;               // [3 faces] x, y, z, minimum
+            float2* range;              // [3 faces] maximum, brick slot (bits)
+        };
+
+        // Forward pass, and both characteristics of the correction: they need the same field and start
+        // from the same velocity, so each face is traced back and forth once.  Bound by instruction
+        // issue and L1 gathers (ten trilinear samples, four locations per face): 0.57 ms for the 4.3 M
+        // faces of a 1.3 M-cell grid on three levels.  With the samples on the extended lattices and the
+        // traces shared, a whole advection takes 1.0 instead of 19.8 ms there (correction 0.14,
+        // extensions 0.2 ms).
+        __global__ void __launch_bounds__(256) mac_forward_kernel(MacView m, Faces f, Links links, int64_t total, float dt, Out out, Feet feet)
         {
             const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
             if (q >= total) return;
@@ -335,56 +466,64 @@ namespace pcfd
             const int64_t at = axis_face(m.bs, c, slot, i, j, k);
             const float current = f.c[c][at];
             const uint8_t link = links.c[c][at];
+            float4 foot = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            float2 range = make_float2(0.0f, __int_as_float(-1));
             float result;
             if (link & 0x40) result = band_update(m, f, links.c, level, slot, rec, c, i, j, k, current, link, dt);
             else
             {
-                float x, y, z;
-                face_point(rec, c, i, j, k, x, y, z);
-                trace(m, f, level, slot, rec, x, y, z, dt);
-                result = sample_finest(m, f, c, x, y, z, current, nullptr, nullptr);
+                float px, py, pz;
+                face_point(rec, c, i, j, k, px, py, pz);
+                const Home home = home_of(m, level, slot, rec);
+                float u[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) u[a] = sample(m, f, level, slot, rec, a, px, py, pz);
+                float bx = px, by = py, bz = pz, fx = px, fy = py, fz = pz;
+                trace(m, f, home, u, bx, by, bz, dt);
+                trace(m, f, home, u, fx, fy, fz, -dt);
+                int back_level = -1, forward_level = -1, owner_level = -1;
+                const int back = locate_near(m, home, bx, by, bz, back_level);
+                float mn = current, mx = current;
+                result = current;
+                if (back >= 0) result = sample_bounded(m, f, back_level, back, record_of(m, back_level, back), c, bx, by, bz, &mn, &mx);
+                // the reverse correction only when the node and both feet are on this level: across a
+                // 2:1 transition the forward field mixes independently evolved lattices
+                clamp_point(m, px, py, pz);
+                locate_near(m, home, px, py, pz, owner_level);
+                const int ahead = locate_near(m, home, fx, fy, fz, forward_level);
+                foot = make_float4(fx, fy, fz, mn);
+                range = make_float2(mx, __int_as_float(owner_level == level && back_level == level && forward_level == level ? ahead : -1));
             }
             out.c[c][at] = result;
+            const int64_t n = (at + c * (total / 3));
+            feet.foot[n] = foot;
+            feet.range[n] = range;
         }
 
-        __global__ void mac_correct_kernel(MacView m, Faces f, Faces forward, Links links, int64_t total, float dt, Out out)
+        // MacCormack correction, written over the current field (each face is read by its own thread
+        // only); m.ext holds the forward field's lattices.  Covered bricks' faces become 0.
+        __global__ void __launch_bounds__(256) mac_correct_kernel(MacView m, Faces forward, int64_t total, Feet feet, Out current)
         {
             const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
             if (q >= total) return;
             int c, i, j, k;
             int64_t slot;
             decode(q, m.bs, c, slot, i, j, k);
-            if (covered(m, slot)) return;
-            const int level = m.slot_level[slot];
-            const float4 rec = record_of(m, level, slot);
             const int64_t at = axis_face(m.bs, c, slot, i, j, k);
-            const float current = f.c[c][at], phf = forward.c[c][at];
+            if (covered(m, slot)) { current.c[c][at] = 0.0f; return; }
+            const int64_t n = at + c * (total / 3);
+            const float2 range = feet.range[n];
+            const float phf = forward.c[c][at];
+            const int ahead = __float_as_int(range.y);
             float result = phf;
-            if (!(links.c[c][at] & 0x40))
+            if (ahead >= 0)
             {
-                float px, py, pz;
-                face_point(rec, c, i, j, k, px, py, pz);
-                float bx = px, by = py, bz = pz;
-                trace(m, f, level, slot, rec, bx, by, bz, dt);
-                float mn, mx;
-                sample_finest(m, f, c, bx, by, bz, current, &mn, &mx);
-                float fx = px, fy = py, fz = pz;
-                trace(m, f, level, slot, rec, fx, fy, fz, -dt);
-                // the reverse correction only when the node and both feet are on this level: across a
-                // 2:1 transition the forward field mixes independently evolved lattices
-                float ox = px, oy = py, oz = pz;
-                clamp_point(m, ox, oy, oz);
-                int owner_level, back_level, forward_level;
-                locate(m, ox, oy, oz, owner_level);
-                locate(m, bx, by, bz, back_level);
-                locate(m, fx, fy, fz, forward_level);
-                if (owner_level == level && back_level == level && forward_level == level)
-                {
-                    const float phn = sample_finest(m, forward, c, fx, fy, fz, phf, nullptr, nullptr);
-                    result = fmaxf(mn, fminf(mx, phf + 0.5f * (current - phn)));
-                }
+                const int level = m.slot_level[slot];
+                const float4 foot = feet.foot[n];
+                const float phn = sample(m, forward, level, ahead, record_of(m, level, ahead), c, foot.x, foot.y, foot.z);
+                result = fmaxf(foot.w, fminf(range.x, phf + 0.5f * (current.c[c][at] - phn)));
             }
-            out.c[c][at] = result;
+            current.c[c][at] = result;
         }
 
         // ---- LES and diffusion ----
@@ -487,22 +626,22 @@ namespace pcfd
             nut[q] = length * length * magnitude;
         }
 
-        __global__ void mac_diffuse_kernel(MacView m, Faces f, Links links, const float* nut, int64_t total, float nu, float dt, Out out)
+        // Written over the field: neighbours are read from the extended lattices, the face itself by
+        // its own thread only.  Covered bricks' faces become 0.
+        __global__ void __launch_bounds__(256) mac_diffuse_kernel(MacView m, Links links, const float* nut, int64_t total, float nu, float dt, Out out)
         {
             const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
             if (q >= total) return;
             int c, i, j, k;
             int64_t slot;
             decode(q, m.bs, c, slot, i, j, k);
-            if (covered(m, slot)) return;
             const int bs = m.bs;
-            const int level = m.slot_level[slot];
             const int64_t at = axis_face(bs, c, slot, i, j, k);
-            const float current = f.c[c][at];
+            if (covered(m, slot)) { out.c[c][at] = 0.0f; return; }
+            const int level = m.slot_level[slot];
+            const float current = out.c[c][at];
             const uint8_t link = links.c[c][at];
-            auto face_value = [&](int a, int b, int d) {
-                return valid_face(c, bs, a, b, d) ? clamped(f, bs, c, slot, a, b, d) : node_value(m, f, level, slot, c, a, b, d);
-            };
+            auto face_value = [&](int a, int b, int d) { return m.ext[ext_index(c, bs, slot, a, b, d)]; };
             float laplacian = 0, viscosity = nu;
             if (!(link & 0x40))
             {
@@ -570,7 +709,12 @@ namespace pcfd
         DBuf<int> neighbour;
         DBuf<uint32_t> flags;
         DBuf<uint8_t> links[3];
-        DBuf<float> forward[3], out[3], nut;
+        DBuf<float> forward[3], nut;
+        DBuf<int> ext_source, ext_slow;         // extended-lattice nodes: source faces, nodes interpolated on another level
+        int slow_count = 0;
+        DBuf<float> ext;                        // [B][3][ext_size] extended lattices of the field last extended
+        DBuf<float4> foot;                      // [3 faces] forward pass -> correction (Feet)
+        DBuf<float2> range;
         DBuf<unsigned int> maximum;
         bool has_links = false;
     };
@@ -585,7 +729,40 @@ namespace pcfd
         MacView mac_view(System& s)
         {
             MacState& st = mac_state(s);
-            return MacView{locator_view(s), st.neighbour.p, st.flags.p, s.brick_level, s.bs};
+            return MacView{locator_view(s), st.neighbour.p, st.flags.p, s.brick_level, s.bs, st.ext.p};
+        }
+        int64_t ext_total(const System& s) { return int64_t(s.B) * 3 * ext_size(s.bs); }
+        // the lattice nodes' sources (grid only) and the buffers of the extended field
+        void build_extension(System& s)
+        {
+            MacState& st = mac_state(s);
+            const int64_t total = ext_total(s);
+            require(total < (int64_t(1) << 31) && s.faces < (int64_t(1) << 31), "MAC momentum: grid too large");
+            st.ext_source.alloc(size_t(total), false);
+            st.ext.alloc(size_t(total));
+            DBuf<int> count;
+            count.alloc(1);
+            const MacView m = mac_view(s);
+            int* list = nullptr;
+            for (int pass = 0; pass < 2; ++pass)
+            {
+                cuda_check(cudaMemsetAsync(count.p, 0, sizeof(int), s.stream), "clear node count");
+                mac_source_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(m, total, st.ext_source, list, count);
+                cuda_check(cudaMemcpyAsync(&st.slow_count, count.p, sizeof(int), cudaMemcpyDeviceToHost, s.stream), "node count");
+                cuda_check(cudaStreamSynchronize(s.stream), "extended lattice nodes");
+                if (!st.slow_count) break;
+                if (!list) st.ext_slow.alloc(size_t(st.slow_count), false);
+                list = st.ext_slow.p;
+            }
+        }
+        void extend(System& s, const Faces& f)
+        {
+            MacState& st = mac_state(s);
+            const int64_t total = ext_total(s);
+            mac_extend_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(f, ext_size(s.bs), total, st.ext_source, st.ext);
+            if (st.slow_count)
+                mac_extend_slow_kernel<<<blocks_for(st.slow_count, 64), 64, 0, launch_stream(s)>>>(mac_view(s), f, st.slow_count, st.ext_slow,
+                                                                                                  st.ext);
         }
     }
 
@@ -627,9 +804,14 @@ namespace pcfd
         {
             st.links[c].upload(std::vector<uint8_t>(host[c], host[c] + s.faces));
             if (!st.forward[c].n) st.forward[c].alloc(size_t(s.faces));
-            if (!st.out[c].n) st.out[c].alloc(size_t(s.faces));
         }
         if (!st.nut.n) st.nut.alloc(size_t(s.S));
+        if (!st.ext.n)
+        {
+            st.foot.alloc(size_t(s.faces) * 3, false);
+            st.range.alloc(size_t(s.faces) * 3, false);
+            build_extension(s);
+        }
         st.has_links = true;
     }
 
@@ -642,14 +824,13 @@ namespace pcfd
         const Links links{{st.links[0].p, st.links[1].p, st.links[2].p}};
         const int64_t total = int64_t(s.B) * 3 * s.bs * s.bs * (s.bs + 1);
         const Out forward{{st.forward[0].p, st.forward[1].p, st.forward[2].p}};
-        mac_forward_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(m, f, links, total, dt, forward);
+        const Feet feet{st.foot.p, st.range.p};
+        extend(s, f);
+        mac_forward_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(m, f, links, total, dt, forward, feet);
         const Faces fw{{st.forward[0].p, st.forward[1].p, st.forward[2].p}};
-        const Out out{{st.out[0].p, st.out[1].p, st.out[2].p}};
-        mac_correct_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(m, f, fw, links, total, dt, out);
-        float* target[3] = {s.u.p, s.v.p, s.w.p};
-        for (int c = 0; c < 3; ++c)
-            cuda_check(cudaMemcpyAsync(target[c], st.out[c].p, size_t(s.faces) * sizeof(float), cudaMemcpyDeviceToDevice, s.stream),
-                       "commit MAC advection");
+        extend(s, fw);
+        const Out out{{s.u.p, s.v.p, s.w.p}};
+        mac_correct_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(m, fw, total, feet, out);
         cuda_check(cudaGetLastError(), "MAC advection");
     }
 
@@ -661,14 +842,11 @@ namespace pcfd
         const Faces f{{s.u.p, s.v.p, s.w.p}};
         const Links links{{st.links[0].p, st.links[1].p, st.links[2].p}};
         const int64_t cells = int64_t(s.B) * s.bs * s.bs * s.bs;
+        extend(s, f);
         mac_smagorinsky_kernel<<<blocks_for(cells), kThreads, 0, launch_stream(s)>>>(m, f, cells, cs, st.nut.p);
         const int64_t total = int64_t(s.B) * 3 * s.bs * s.bs * (s.bs + 1);
-        const Out out{{st.out[0].p, st.out[1].p, st.out[2].p}};
-        mac_diffuse_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(m, f, links, st.nut.p, total, nu, dt, out);
-        float* target[3] = {s.u.p, s.v.p, s.w.p};
-        for (int c = 0; c < 3; ++c)
-            cuda_check(cudaMemcpyAsync(target[c], st.out[c].p, size_t(s.faces) * sizeof(float), cudaMemcpyDeviceToDevice, s.stream),
-                       "commit MAC diffusion");
+        const Out out{{s.u.p, s.v.p, s.w.p}};
+        mac_diffuse_kernel<<<blocks_for(total), kThreads, 0, launch_stream(s)>>>(m, links, st.nut.p, total, nu, dt, out);
         cuda_check(cudaGetLastError(), "MAC diffusion");
     }
 
