@@ -17,8 +17,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <memory>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace pcfd
@@ -126,6 +128,22 @@ namespace pcfd
         double prolong = 1.0;                   // weight of the next level's correction added here
         int sweeps = 2;                         // smoothing steps before and after the coarse correction
         int chebyshev = 0;                      // 0: damped Jacobi; r >= 2: Chebyshev on [2 / r, 2]
+    };
+
+    // A hierarchy level's rows, parents and members on the host, while it is being built.
+    struct HostRows
+    {
+        int cells = 0;
+        const std::vector<int> *row_offset, *neighbour, *parent, *member_offset, *member;
+        const std::vector<double> *weight, *diagonal;
+    };
+    // The levels at the coarse end of a hierarchy that run as one cluster launch (stage_tail.cu):
+    // those from `first` of the chain on, or none (first < 0).
+    struct TailPlan;
+    struct StageTail
+    {
+        int first = -1;
+        std::shared_ptr<TailPlan> plan;
     };
 
     struct Scalars;   // device scalar block for the Krylov recurrences
@@ -248,6 +266,7 @@ namespace pcfd
         DBuf<double> fine_residual;             // [S] r - A_orth z before the first restriction
         FineSmoother fine;
         cudaGraphExec_t mg_graph64 = nullptr, mg_graph32 = nullptr, mg_graph_composite = nullptr;   // captured hierarchies
+        StageTail mg_tail64, mg_tail32, composite_tail;   // their small levels as one launch
         int64_t mg_graph64_launches = 0, mg_graph32_launches = 0, mg_graph_composite_launches = 0;
         bool composite_fp32 = false;            // composite stages in float
         DBuf<float> diagonal32;
@@ -409,6 +428,13 @@ namespace pcfd
     template <class T> void fine_preconditioner(System& s, const double* r, double* z, std::vector<MgLevel<T>>& levels);
     template <class T> void multigrid_levels(System& s, std::vector<MgLevel<T>>& levels);
     void build_composite(System& s, const pcfd_topology& t);
+    // smoothing steps of a level as (c1, c2): d = c1 d + c2 D^-1 (b - A x), x += d (solver.cu)
+    std::vector<std::pair<double, double>> smoothing_steps(int chebyshev, int sweeps);
+    // stage_tail.cu; coarsest_sweeps, omega: the coarsest level's damped Jacobi without an inverse
+    void plan_tail(std::vector<MgLevel<double>>& levels, const std::vector<HostRows>& rows, int coarsest_sweeps, double omega, StageTail& tail);
+    void plan_tail(std::vector<MgLevel<float>>& levels, const std::vector<HostRows>& rows, int coarsest_sweeps, double omega, StageTail& tail);
+    void launch_tail(System& s, MgLevel<double>& level, const StageTail& tail);
+    void launch_tail(System& s, MgLevel<float>& level, const StageTail& tail);
     void composite_levels(System& s);                 // V-cycle below the fine level, composite chain
     int64_t krylov_sweep_entries(const System& s);    // vector entries the Krylov block kernels sweep
     void composite_preconditioner(System& s, const double* r, double* z);   // smoother.cu

@@ -1003,7 +1003,6 @@ namespace pcfd
         FineSmoother& f = s.fine;
         MgLevel<TC>& base = levels.front();
         auto coarse = [&](auto* zz, auto* rr) {
-            cuda_check(cudaMemsetAsync(base.x, 0, size_t(base.cells) * sizeof(TC), s.stream), "clear base correction");
             restrict_residual(s, zz, rr);
             gather_base_kernel<TC><<<blocks_for(base.cells), kThreads, 0, launch_stream(s)>>>(
                 base.cells, f.gather_offset, f.gather_entry, f.partial, f.deferred_residual, base.rhs);
@@ -1142,7 +1141,6 @@ namespace pcfd
                 view(s), s.active_bricks, z, r, res, f.t.p, nullptr, nullptr, f.damping.p);
             finish<2, double, double, TC, 0>(s, z, r, res, static_cast<const TC*>(nullptr), f.t.p);
             gather_first<TC, double>(s, res, first);
-            cuda_check(cudaMemsetAsync(first.x, 0, size_t(first.cells) * sizeof(TC), s.stream), "clear stage correction");
             composite_levels(s);
             sweep<double, double, TC, 2>(s, z, r, a, first.x.p, schedule ? 2 : -1);
             sweep<double, double, TC, 0>(s, a, r, z, nullptr, schedule ? 3 : -1);
@@ -1163,7 +1161,6 @@ namespace pcfd
                 view(s), s.active_bricks, b, r32, res, f.t32.p, nullptr, nullptr, f.damping32.p);
             finish<2, float, float, float, 0>(s, b, r32, res, static_cast<const float*>(nullptr), f.t32.p);
             gather_first<float, float>(s, res, first);
-            cuda_check(cudaMemsetAsync(first.x, 0, size_t(first.cells) * sizeof(float), s.stream), "clear stage correction");
             composite_levels(s);
             sweep<float, float, float, 2>(s, b, r32, a, first.x.p, 2);
             sweep<float, double, float, 0>(s, a, r32, z, nullptr, 3);
@@ -1206,7 +1203,6 @@ namespace pcfd
         }
         else if (stage == 2)
         {
-            cuda_check(cudaMemsetAsync(base.x, 0, size_t(base.cells) * sizeof(double), s.stream), "clear base correction");
             multigrid_levels(s, levels);
         }
         else

@@ -4,9 +4,9 @@
 // damped Jacobi (omega 2/3) on the finest composite graph around a Galerkin-style aggregation
 // hierarchy built on the level-0 Cartesian lattice (setup :857-1069): every active DOF is summed
 // into its level-0 cell, coarse levels aggregate 2x2x2 lattice cells through union-find, and the
-// coarsest level (<= 512 cells or 8 levels) takes 96 Jacobi sweeps.  The coarsest sweeps run
-// inside ONE CTA here (grid-wide launch loop of the reference removed; results are identical
-// because a Jacobi sweep is order-independent per row).
+// coarsest level (<= 512 cells or 8 levels) takes 96 Jacobi sweeps.  The small levels, the
+// coarsest sweeps included, run as one cluster launch (stage_tail.cu); a Jacobi sweep is
+// order-independent per row, so the results are those of separate launches.
 //
 // Outer solvers: FP64 PCG with periodic true-residual replacement (reference :1267-1353) for an
 // orthogonal operator and flexible GCRO/LGMRES(24) with 3 recycled vectors (reference :1390-1698)
@@ -164,6 +164,14 @@ namespace pcfd
             rest_coefficient.upload(rest_value);
         }
 
+        std::vector<HostRows> host_rows(const std::vector<GraphLevel>& levels)
+        {
+            std::vector<HostRows> rows;
+            for (const GraphLevel& l : levels)
+                rows.push_back(HostRows{l.cells, &l.row_offset, &l.neighbour, &l.parent, &l.member_offset, &l.member, &l.weight, &l.diagonal});
+            return rows;
+        }
+
         double connection_factor(const pcfd_connections& c, int e)
         {
             const double f = c.orthogonal_gradient_factor[e];
@@ -313,6 +321,30 @@ namespace pcfd
         }
     }
 
+    namespace
+    {
+        constexpr double kOmega = 2.0 / 3.0;
+        constexpr int kCoarsestSweeps = 96;
+    }
+
+    std::vector<std::pair<double, double>> smoothing_steps(int chebyshev, int sweeps)
+    {
+        std::vector<std::pair<double, double>> steps(size_t(sweeps), {0.0, kOmega});
+        if (chebyshev < 2) return steps;
+        // Chebyshev polynomial smoothing on [2 / ratio, 2] (D^-1 A of a diagonally dominant Galerkin
+        // level has its spectrum in (0, 2])
+        const double hi = 2.0, lo = hi / chebyshev, theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
+        double rho = 1.0 / sigma;
+        for (int k = 0; k < sweeps; ++k)
+        {
+            if (k == 0) { steps[0] = {0.0, 1.0 / theta}; continue; }
+            const double next = 1.0 / (2.0 * sigma - rho);
+            steps[size_t(k)] = {next * rho, 2.0 * next / delta};
+            rho = next;
+        }
+        return steps;
+    }
+
     // The reference's lattice multigrid (its setup: amr_pressure.cu:915-1069), built here as
     // Galerkin levels: the active DOFs summed into their level-0 Cartesian cells
     // (preconditioner_aggregate), then block aggregates of 2x2x2 lattice cells while the level
@@ -372,7 +404,9 @@ namespace pcfd
         {
             s.mg32.resize(levels.size());
             for (size_t l = 0; l < levels.size(); ++l) upload_level(s.mg32[l], levels[l]);
+            plan_tail(s.mg32, host_rows(levels), kCoarsestSweeps, kOmega, s.mg_tail32);
         }
+        plan_tail(s.mg64, host_rows(levels), kCoarsestSweeps, kOmega, s.mg_tail64);
     }
 
     // ==================================================================================
@@ -697,6 +731,8 @@ namespace pcfd
                 upload_brick_rows<double, double>(s.inter64.front(), stages[0], brick_neighbour, [](double w) { return w; },
                                                   s.inter64.front().rest_coefficient);
         }
+        if (s.composite_fp32) plan_tail(s.inter32, host_rows(stages), kCoarsestSweeps, kOmega, s.composite_tail);
+        else plan_tail(s.inter64, host_rows(stages), kCoarsestSweeps, kOmega, s.composite_tail);
         s.composite = true;
     }
 
@@ -705,8 +741,6 @@ namespace pcfd
     // ==================================================================================
     namespace
     {
-        constexpr double kOmega = 2.0 / 3.0;
-
         __global__ void precondition_kernel(const double* r, double* z, const double* diag, const uint8_t* active, int64_t n, double omega)
         {
             const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -734,15 +768,21 @@ namespace pcfd
         __device__ inline double coefficient_value(__half c) { return double(__half2float(c)); }
 
         template <class T, class TK = T>
-        __global__ void algebraic_jacobi_kernel(const T* rhs, const T* x, T* next, const int* row_offset, const int* neighbour,
-                                                const TK* coefficient, const T* diag, int cells, T omega)
+        __global__ void __launch_bounds__(256) algebraic_jacobi_kernel(const T* __restrict__ rhs, const T* __restrict__ x,
+            T* __restrict__ next, const int* __restrict__ row_offset, const int* __restrict__ neighbour,
+            const TK* __restrict__ coefficient, const T* __restrict__ diag, int cells, T omega)
         {
+            chain_wait();
+            chain_release();
             const int q = blockIdx.x * blockDim.x + threadIdx.x;
             if (q >= cells) return;
-            if (!(diag[q] > T(0))) { next[q] = T(0); return; }
-            double Ax = double(diag[q]) * double(x[q]);
-            for (int e = row_offset[q]; e < row_offset[q + 1]; ++e) Ax -= coefficient_value(coefficient[e]) * double(x[neighbour[e]]);
-            next[q] = x[q] + omega * T((double(rhs[q]) - Ax) / double(diag[q]));
+            const T dq = diag[q], xq = x[q], bq = rhs[q];
+            const int e0 = row_offset[q], e1 = row_offset[q + 1];
+            if (!(dq > T(0))) { next[q] = T(0); return; }
+            double Ax = double(dq) * double(xq);
+#pragma unroll 4
+            for (int e = e0; e < e1; ++e) Ax -= coefficient_value(coefficient[e]) * double(x[neighbour[e]]);
+            next[q] = xq + omega * T((double(bq) - Ax) / double(dq));
         }
         // x = inverse * rhs on a coarsest level (one warp per row, FP64 accumulation)
         template <class T>
@@ -783,9 +823,9 @@ namespace pcfd
             d[q] = dn;
             next[q] = xq + dn;
         }
-        // The first Chebyshev step from x = 0 (every pre-smoothing of a stage correction): the
-        // residual is the right-hand side, so d = c2 D^-1 rhs and next = 0 + d without reading the
-        // matrix or the iterate; the same values as the general step.
+        // The first step from x = 0 (every pre-smoothing of a correction; damped Jacobi with
+        // c2 = omega): the residual is the right-hand side, so d = c2 D^-1 rhs and next = 0 + d without
+        // reading the matrix or the iterate; the same values as the general step.
         template <class T>
         __global__ void __launch_bounds__(256) chebyshev_zero_start_kernel(const T* __restrict__ rhs, T* __restrict__ next,
                                                                            T* __restrict__ d, const T* __restrict__ diag, int cells, T c2)
@@ -977,72 +1017,62 @@ namespace pcfd
                 for (int q = threadIdx.x; q < cells; q += blockDim.x) x[q] = temporary[q];
         }
 
-        // One V-cycle from chain[index] down: level.sweeps Jacobi sweeps, residual, restriction,
-        // the coarser levels, the weighted prolongation (chain[index]->prolong), level.sweeps
-        // sweeps; the last level takes 96 sweeps (in one CTA when it fits).
+        // One V-cycle from chain[index] down: level.sweeps smoothing steps from x = 0, residual,
+        // restriction, the coarser levels, the weighted prolongation (chain[index]->prolong),
+        // level.sweeps steps; the last level applies its explicit inverse or takes 96 sweeps (in one CTA
+        // when it fits).  Levels from tail.first on run as one cluster launch.
         template <class T>
-        void mg_level(System& s, MgLevel<T>* const* chain, int count, int index)
+        void mg_level(System& s, MgLevel<T>* const* chain, int count, int index, const StageTail& tail)
         {
             MgLevel<T>& level = *chain[index];
+            if (index == tail.first)
+            {
+                launch_tail(s, level, tail);
+                return;
+            }
             const T omega = T(kOmega);
-            // from_zero: x is 0 on entry (pre-smoothing of a correction), so the first Chebyshev
-            // step needs neither the matrix nor x
+            // from_zero: the pre-smoothing of a correction, whose first step needs neither the matrix
+            // nor x; the Chebyshev direction lives in level.residual
             auto smooth = [&](int sweeps, bool from_zero) {
-                if (level.chebyshev >= 2)
+                const std::vector<std::pair<double, double>> steps = smoothing_steps(level.chebyshev, sweeps);
+                for (int sweep = 0; sweep < sweeps; ++sweep)
                 {
-                    // Chebyshev polynomial smoothing on [2 / ratio, 2] (D^-1 A of a diagonally dominant
-                    // Galerkin level has its spectrum in (0, 2]); the direction lives in level.residual
-                    const double hi = 2.0, lo = hi / level.chebyshev;
-                    const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
-                    double rho = 1.0 / sigma;
-                    for (int sweep = 0; sweep < sweeps; ++sweep)
+                    const T c1 = T(steps[size_t(sweep)].first), c2 = T(steps[size_t(sweep)].second);
+                    if (from_zero && sweep == 0)
                     {
-                        double c1 = 0.0, c2 = 1.0 / theta;
-                        if (sweep)
-                        {
-                            const double next = 1.0 / (2.0 * sigma - rho);
-                            c1 = next * rho;
-                            c2 = 2.0 * next / delta;
-                            rho = next;
-                        }
-                        if (from_zero && sweep == 0)
-                        {
-                            launch_chained(s, chebyshev_zero_start_kernel<T>, blocks_for(level.cells), kThreads,
-                                level.rhs, level.temporary, level.residual, level.diagonal, level.cells, T(c2));
-                            std::swap(level.x.p, level.temporary.p);
-                            continue;
-                        }
+                        launch_chained(s, chebyshev_zero_start_kernel<T>, blocks_for(level.cells), kThreads,
+                            level.rhs, level.temporary, level.residual, level.diagonal, level.cells, c2);
+                        std::swap(level.x.p, level.temporary.p);
+                        continue;
+                    }
+                    if (level.chebyshev >= 2)
+                    {
                         // the first composite stage's full steps are the profiled stage-smoothing region
                         ProfileScope scope(s, index == 0 && s.composite ? PCFD_PROFILE_STAGE_SMOOTH : -1);
                         if (level.brick_rows.p && level.coefficient16.p)
                             launch_chained(s, brick_stage_chebyshev_kernel<T, __half>, blocks_for(level.cells), kThreads,
                                 level.rhs, level.x, level.temporary, level.residual, brick_stage16(level), level.diagonal, level.cells,
-                                T(c1), T(c2), sweep == 0 ? 1 : 0);
+                                c1, c2, sweep == 0 ? 1 : 0);
                         else if (level.brick_rows.p)
                             launch_chained(s, brick_stage_chebyshev_kernel<T, T>, blocks_for(level.cells), kThreads,
                                 level.rhs, level.x, level.temporary, level.residual, brick_stage(level), level.diagonal, level.cells,
-                                T(c1), T(c2), sweep == 0 ? 1 : 0);
+                                c1, c2, sweep == 0 ? 1 : 0);
                         else if (level.coefficient16.p)
                             launch_chained(s, algebraic_chebyshev_kernel<T, __half>, blocks_for(level.cells), kThreads,
                                 level.rhs, level.x, level.temporary, level.residual, level.row_offset, level.neighbour,
-                                reinterpret_cast<const __half*>(level.coefficient16.p), level.diagonal, level.cells, T(c1), T(c2),
+                                reinterpret_cast<const __half*>(level.coefficient16.p), level.diagonal, level.cells, c1, c2,
                                 sweep == 0 ? 1 : 0);
                         else
                             launch_chained(s, algebraic_chebyshev_kernel<T, T>, blocks_for(level.cells), kThreads,
                                 level.rhs, level.x, level.temporary, level.residual, level.row_offset, level.neighbour, level.coefficient,
-                                level.diagonal, level.cells, T(c1), T(c2), sweep == 0 ? 1 : 0);
-                        std::swap(level.x.p, level.temporary.p);
+                                level.diagonal, level.cells, c1, c2, sweep == 0 ? 1 : 0);
                     }
-                    return;
-                }
-                for (int sweep = 0; sweep < sweeps; ++sweep)
-                {
-                    if (level.coefficient16.p)
-                        algebraic_jacobi_kernel<T, __half><<<blocks_for(level.cells), kThreads, 0, launch_stream(s)>>>(
+                    else if (level.coefficient16.p)
+                        launch_chained(s, algebraic_jacobi_kernel<T, __half>, blocks_for(level.cells), kThreads,
                             level.rhs, level.x, level.temporary, level.row_offset, level.neighbour,
                             reinterpret_cast<const __half*>(level.coefficient16.p), level.diagonal, level.cells, omega);
                     else
-                        algebraic_jacobi_kernel<T, T><<<blocks_for(level.cells), kThreads, 0, launch_stream(s)>>>(
+                        launch_chained(s, algebraic_jacobi_kernel<T, T>, blocks_for(level.cells), kThreads,
                             level.rhs, level.x, level.temporary, level.row_offset, level.neighbour, level.coefficient,
                             level.diagonal, level.cells, omega);
                     std::swap(level.x.p, level.temporary.p);
@@ -1054,10 +1084,13 @@ namespace pcfd
                     launch_chained(s, dense_apply_kernel<T>, blocks_for(int64_t(level.cells) * 32), kThreads, level.inverse, level.rhs,
                                                                                                               level.x, level.cells);
                 else if (level.cells <= 4096)
+                {
+                    cuda_check(cudaMemsetAsync(level.x, 0, size_t(level.cells) * sizeof(T), s.stream), "clear coarse correction");
                     coarse_jacobi_kernel<T, 4><<<1, 1024, 0, launch_stream(s)>>>(level.rhs, level.x, level.temporary, level.row_offset,
-                        level.neighbour, level.coefficient, level.diagonal, level.cells, omega, 96);
+                        level.neighbour, level.coefficient, level.diagonal, level.cells, omega, kCoarsestSweeps);
+                }
                 else
-                    smooth(96, true);
+                    smooth(kCoarsestSweeps, true);
                 return;
             }
             smooth(level.sweeps, true);
@@ -1077,34 +1110,23 @@ namespace pcfd
             MgLevel<T>& coarse = *chain[index + 1];
             launch_chained(s, restrict_gather_kernel<T>, blocks_for(coarse.cells), kThreads,
                 level.restrict_offset, level.restrict_dof, level.residual, coarse.cells, coarse.rhs);
-            // the coarse correction starts from 0; only a first step that reads x needs it cleared
-            const bool coarsest = index + 2 == count;
-            const bool writes_x_first = coarse.chebyshev >= 2 ? !(coarsest && !coarse.inverse.p && coarse.cells <= 4096)
-                                                              : (coarsest && coarse.inverse.p);
-            if (!writes_x_first)
-                cuda_check(cudaMemsetAsync(coarse.x, 0, size_t(coarse.cells) * sizeof(T), s.stream), "clear coarse correction");
-            mg_level(s, chain, count, index + 1);
+            mg_level(s, chain, count, index + 1, tail);
             launch_chained(s, prolong_add_kernel<T>, blocks_for(level.cells), kThreads, level.aggregate, level.cells, coarse.x, level.x,
                                                                                              T(level.prolong));
             smooth(level.sweeps, false);
         }
 
-        template <class T> void mg_level(System& s, std::vector<MgLevel<T>>& levels, int index)
-        {
-            std::vector<MgLevel<T>*> chain;
-            for (MgLevel<T>& level : levels) chain.push_back(&level);
-            mg_level(s, chain.data(), int(chain.size()), index);
-        }
-
         // Runs mg_level over `chain` through a CUDA graph captured on first use (the chain and its
         // buffers are fixed for the system's lifetime).
         template <class T>
-        void run_captured(System& s, std::vector<MgLevel<T>*>& chain, cudaGraphExec_t& exec, int64_t& nodes)
+        void run_captured(System& s, std::vector<MgLevel<T>*>& chain, const StageTail& tail, cudaGraphExec_t& exec, int64_t& nodes)
         {
             // uncaptured while the stage-smoothing region is profiled: its launches get event pairs
+            // (and a first stage small enough for the cluster launch runs as launches of its own)
             if (!s.stream || s.profile_region == PCFD_PROFILE_STAGE_SMOOTH)
             {
-                mg_level(s, chain.data(), int(chain.size()), 0);
+                const bool apart = s.profile_region == PCFD_PROFILE_STAGE_SMOOTH && tail.first == 0;
+                mg_level(s, chain.data(), int(chain.size()), 0, apart ? StageTail{} : tail);
                 return;
             }
             if (!exec)
@@ -1114,7 +1136,7 @@ namespace pcfd
                 cudaGraph_t graph = nullptr;
                 try
                 {
-                    mg_level(s, chain.data(), int(chain.size()), 0);
+                    mg_level(s, chain.data(), int(chain.size()), 0, tail);
                 }
                 catch (...)
                 {
@@ -1134,14 +1156,15 @@ namespace pcfd
         }
 
         template <class T>
-        void coarse_correction(System& s, std::vector<MgLevel<T>>& levels, const double* r, double* z)
+        void coarse_correction(System& s, std::vector<MgLevel<T>>& levels, const StageTail& tail, const double* r, double* z)
         {
             MgLevel<T>& base = levels.front();
-            cuda_check(cudaMemsetAsync(base.x, 0, size_t(base.cells) * sizeof(T), s.stream), "clear base correction");
             launch_apply(s, z, s.t, true);
             restrict_difference_kernel<T><<<blocks_for(base.cells), kThreads, 0, launch_stream(s)>>>(
                 s.base_restrict_offset, s.base_restrict_dof, r, s.t, base.cells, base.rhs);
-            mg_level(s, levels, 0);
+            std::vector<MgLevel<T>*> chain;
+            for (MgLevel<T>& level : levels) chain.push_back(&level);
+            mg_level(s, chain.data(), int(chain.size()), 0, tail);
             prolong_aggregate_kernel<T><<<blocks_for(s.S), kThreads, 0, launch_stream(s)>>>(s.aggregate, s.active, s.S, s.base_offset,
                                                                                   s.base_cells, base.x, z, s.mg_prolong_scale);
         }
@@ -1157,8 +1180,8 @@ namespace pcfd
         }
         else if (stage == 1 && !s.mg64.empty())
         {
-            if (s.mg_precision == PCFD_MG_FP32 && !s.mg32.empty()) coarse_correction(s, s.mg32, r, z);
-            else coarse_correction(s, s.mg64, r, z);
+            if (s.mg_precision == PCFD_MG_FP32 && !s.mg32.empty()) coarse_correction(s, s.mg32, s.mg_tail32, r, z);
+            else coarse_correction(s, s.mg64, s.mg_tail64, r, z);
         }
         else if (stage == 2 && !s.mg64.empty())
             for (int sweep = 0; sweep < 2; ++sweep)
@@ -1177,7 +1200,7 @@ namespace pcfd
         const bool fp32 = std::is_same<T, float>::value;
         std::vector<MgLevel<T>*> chain;
         for (MgLevel<T>& level : levels) chain.push_back(&level);
-        run_captured(s, chain, fp32 ? s.mg_graph32 : s.mg_graph64, fp32 ? s.mg_graph32_launches : s.mg_graph64_launches);
+        run_captured(s, chain, fp32 ? s.mg_tail32 : s.mg_tail64, fp32 ? s.mg_graph32 : s.mg_graph64, fp32 ? s.mg_graph32_launches : s.mg_graph64_launches);
     }
 
     // composite chain: the stage levels (FP32 or FP64), the last one the coarsest
@@ -1187,12 +1210,12 @@ namespace pcfd
         {
             std::vector<MgLevel<float>*> chain;
             for (MgLevel<float>& level : s.inter32) chain.push_back(&level);
-            run_captured(s, chain, s.mg_graph_composite, s.mg_graph_composite_launches);
+            run_captured(s, chain, s.composite_tail, s.mg_graph_composite, s.mg_graph_composite_launches);
             return;
         }
         std::vector<MgLevel<double>*> chain;
         for (MgLevel<double>& level : s.inter64) chain.push_back(&level);
-        run_captured(s, chain, s.mg_graph_composite, s.mg_graph_composite_launches);
+        run_captured(s, chain, s.composite_tail, s.mg_graph_composite, s.mg_graph_composite_launches);
     }
 
     // Algorithmic bytes of one step of the first composite stage's smoothing, each array read
