@@ -646,7 +646,9 @@ namespace pcfd
             o[1] = pack8(zero);
             target[i] = ht[src] * target_scale;
             mask[i] = hm[src];
-            if (hm[src]) atomicAdd(count, 1.0f);
+            // one add per warp (a warp's 32 voxels lie in one sample): 49 us for 64 samples with one per voxel
+            const unsigned on = __ballot_sync(0xffffffffu, hm[src] != 0);
+            if ((threadIdx.x & 31) == 0 && on) atomicAdd(count, float(__popc(on)));
         }
 
         // head forward + backward: zhat, loss, dhead, G4 = bf16(dz * head * [d0 > 0])
@@ -683,10 +685,19 @@ namespace pcfd
                 l += __shfl_xor_sync(0xffffffffu, l, o);
                 for (int c = 0; c < 16; ++c) part[c] += __shfl_xor_sync(0xffffffffu, part[c], o);
             }
+            // a CTA's warps in order, then one add per CTA and sum
+            __shared__ float sums[kThreads / 32][17];
             if ((threadIdx.x & 31) == 0)
             {
-                atomicAdd(loss, l);
-                for (int c = 0; c < 16; ++c) atomicAdd(&dhead[c], part[c]);
+                for (int c = 0; c < 16; ++c) sums[threadIdx.x >> 5][c] = part[c];
+                sums[threadIdx.x >> 5][16] = l;
+            }
+            __syncthreads();
+            if (threadIdx.x < 17)
+            {
+                float total = 0;
+                for (int w = 0; w < kThreads / 32; ++w) total += sums[w][threadIdx.x];
+                atomicAdd(threadIdx.x < 16 ? &dhead[threadIdx.x] : loss, total);
             }
         }
 
@@ -725,58 +736,116 @@ namespace pcfd
             G[i] = __float2bfloat16_rn(__bfloat162float(act[i]) > 0 ? S[i] + 0.125f * parent : 0.0f);
         }
 
-        // dW[t][co][ci] += sum_b sum_v G[b][v][co] * src[b][v + shift_t][ci] (FP32, CUDA cores).
-        // Block: 256 threads, each owning a 4 (co) x 4 (ci) block of one tap; blockIdx.y walks a
-        // chunk of samples, staging the padded source and G of one sample at a time.
-        template <int N>
-        __global__ void __launch_bounds__(256) weight_grad_kernel(ConvSource s, const bf16* G, int cout, int samples, int chunk, float* dW)
+        // dW[t][co][ci] += sum_b sum_v G[b][v][co] * src[b][v + shift_t][ci]: per tap a (cout x voxels) by
+        // (voxels x channels) product with K = the voxels, on m16n8k16 tensor-core tiles (BF16 operands,
+        // FP32 sums).  mma.sync rather than tcgen05: the operand rows are voxels shifted by the tap, which
+        // ldmatrix gathers row by row from the padded brick as it lies, and M = cout of 16 to 64 would fill
+        // an eighth to a half of a 128-row tcgen05 tile.  A CTA stages kStage samples at a time
+        // (padded source and G, rows 16 bytes apart from a multiple of the bank width, so that the
+        // eight rows of a matrix fall on distinct banks); its eight warps hold two taps
+        // each, all of cout x channels in registers, and add them to dW once per CTA.
+        // Bound by staging and the final adds: 64 samples of the 8^3 layers take a few us of MMAs.
+        // CUDA-core form: 327 us per 8^3 layer and 54 per 4^3 layer at 64 samples (56 to 108 CTAs, one
+        // shared-memory read per two FMAs); a whole forward and backward pass on 64 samples went from
+        // 1,766 to 600 us with this kernel and the batched counts and sums of the loss kernels.
+        __device__ inline void load_matrices(uint32_t (&r)[4], const void* row)
         {
-            constexpr int XP = N + 2, P = XP * XP * XP, V = N * N * N;
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(row)) : "memory");
+        }
+        __device__ inline void mma_tile(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+        {
+            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+        }
+        template <int N> __host__ __device__ constexpr int wgrad_stage() { return N == 8 ? 1 : N == 4 ? 2 : 4; }   // K = 512, 128, 32 voxels
+        template <int N, int COUT, int C>
+        __global__ void __launch_bounds__(256) weight_grad_kernel(ConvSource s, const bf16* G, int samples, int chunk, float* dW)
+        {
+            constexpr int XP = N + 2, P = XP * XP * XP, V = N * N * N, kStage = wgrad_stage<N>();
+            constexpr int XR = C + 8, GR = COUT + 8;        // row strides
+            constexpr int MT = COUT / 16, NT = C / 8;
             extern __shared__ __align__(16) uint8_t wsm[];
-            const int C = s.channels;
-            bf16* xs = reinterpret_cast<bf16*>(wsm);        // [P][C]
-            bf16* gs = xs + P * C;                          // [V][cout]
-            const int cb = cout / 4, ib = C / 4;
-            const int e = blockIdx.x * 256 + threadIdx.x;
-            const bool owner = e < 27 * cb * ib;
-            const int tap = owner ? e / (cb * ib) : 0, co0 = owner ? 4 * ((e / ib) % cb) : 0, ci0 = owner ? 4 * (e % ib) : 0;
-            const int shift = ((tap / 9) - 1) * XP * XP + ((tap / 3) % 3 - 1) * XP + (tap % 3) - 1;
-            float acc[16];
-            for (int k = 0; k < 16; ++k) acc[k] = 0;
-            const int first = blockIdx.y * chunk, last = min(samples, first + chunk);
-            for (int b = first; b < last; ++b)
+            bf16* xs = reinterpret_cast<bf16*>(wsm);        // [kStage][P][XR]
+            bf16* gs = xs + kStage * P * XR;                // [kStage * V][GR]
+            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            for (int i = threadIdx.x; i < kStage * P * XR / 8; i += 256) reinterpret_cast<uint4*>(xs)[i] = make_uint4(0, 0, 0, 0);
+            const int first = blockIdx.x * chunk, last = min(samples, first + chunk);
+            // blockIdx.y 0: taps 0..15, 1: taps 16..26, two per warp
+            constexpr int kTaps = 2;
+            const int tap0 = 16 * int(blockIdx.y) + kTaps * warp, taps = min(kTaps, 27 - tap0);
             {
-                __syncthreads();
-                for (int i = threadIdx.x; i < P * C / 8; i += 256) reinterpret_cast<uint4*>(xs)[i] = make_uint4(0, 0, 0, 0);
-                __syncthreads();
-                for (int i = threadIdx.x; i < V * (C / 8); i += 256)
+                float acc[kTaps][MT][NT][4] = {};
+                int shift[kTaps];
+#pragma unroll
+                for (int k = 0; k < kTaps; ++k)
                 {
-                    const int v = i / (C / 8), c0 = 8 * (i % (C / 8));
-                    const int x = v % N, y = (v / N) % N, z = v / (N * N);
-                    reinterpret_cast<uint4*>(xs + (((z + 1) * XP + y + 1) * XP + x + 1) * C + c0)[0] = load_source<N>(s, b, x, y, z, c0);
+                    const int tap = min(26, tap0 + k);
+                    shift[k] = ((tap / 9) - 1) * XP * XP + ((tap / 3) % 3 - 1) * XP + (tap % 3) - 1;
                 }
-                for (int i = threadIdx.x; i < V * cout / 8; i += 256)
-                    reinterpret_cast<uint4*>(gs)[i] = reinterpret_cast<const uint4*>(G + int64_t(b) * V * cout)[i];
-                __syncthreads();
-                if (!owner) continue;
-                for (int v = 0; v < V; ++v)
+                for (int b = first; b < last; b += kStage)
                 {
-                    const int x = v % N, y = (v / N) % N, z = v / (N * N);
-                    const int pos = ((z + 1) * XP + y + 1) * XP + x + 1 + shift;
-                    float g[4], xv[4];
-                    for (int k = 0; k < 4; ++k)
+                    __syncthreads();
+                    const int here = min(kStage, last - b);
+                    for (int i = threadIdx.x; i < kStage * V * (C / 8); i += 256)
                     {
-                        g[k] = __bfloat162float(gs[v * cout + co0 + k]);
-                        xv[k] = __bfloat162float(xs[pos * C + ci0 + k]);
+                        const int c0 = 8 * (i % (C / 8)), v = (i / (C / 8)) % V, k = i / (C / 8) / V;
+                        const int x = v % N, y = (v / N) % N, z = v / (N * N);
+                        reinterpret_cast<uint4*>(xs + (k * P + ((z + 1) * XP + y + 1) * XP + x + 1) * XR + c0)[0] =
+                            k < here ? load_source<N>(s, b + k, x, y, z, c0) : make_uint4(0, 0, 0, 0);
                     }
-                    for (int a = 0; a < 4; ++a)
-                        for (int c = 0; c < 4; ++c) acc[4 * a + c] += g[a] * xv[c];
+                    for (int i = threadIdx.x; i < kStage * V * (COUT / 8); i += 256)
+                    {
+                        const int c0 = 8 * (i % (COUT / 8)), v = i / (COUT / 8);
+                        reinterpret_cast<uint4*>(gs + v * GR + c0)[0] =
+                            v / V < here ? *reinterpret_cast<const uint4*>(G + (int64_t(b) * V + v) * COUT + c0) : make_uint4(0, 0, 0, 0);
+                    }
+                    __syncthreads();
+                    if (taps > 0)
+                        for (int k0 = 0; k0 < kStage * V; k0 += 16)
+                        {
+                            // A (cout x 16 voxels) from G rows, B (16 voxels x channels) from shifted source rows
+                            uint32_t a[MT][4];
+                            const int ar = k0 + (lane & 7) + ((lane >> 4) << 3), ac = ((lane >> 3) & 1) << 3;
+#pragma unroll
+                            for (int m = 0; m < MT; ++m) load_matrices(a[m], gs + ar * GR + 16 * m + ac);
+                            const int br = k0 + (lane & 7) + (((lane >> 3) & 1) << 3), bc = (lane >> 4) << 3;
+                            const int v = br % V, sample = br / V;
+                            const int pos = sample * P + ((v / (N * N) + 1) * XP + (v / N) % N + 1) * XP + v % N + 1;
+#pragma unroll
+                            for (int k = 0; k < kTaps; ++k)
+#pragma unroll
+                                for (int n = 0; n < NT; n += 2)
+                                {
+                                    uint32_t bm[4];
+                                    load_matrices(bm, xs + (pos + shift[k]) * XR + 8 * n + bc);
+#pragma unroll
+                                    for (int m = 0; m < MT; ++m)
+                                    {
+                                        mma_tile(acc[k][m][n], a[m], bm[0], bm[1]);
+                                        mma_tile(acc[k][m][n + 1], a[m], bm[2], bm[3]);
+                                    }
+                                }
+                        }
+                }
+#pragma unroll
+                for (int k = 0; k < kTaps; ++k)
+                {
+                    if (k >= taps) continue;
+                    float* out = dW + int64_t(tap0 + k) * COUT * C;
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
+#pragma unroll
+                        for (int n = 0; n < NT; ++n)
+                        {
+                            const int co = 16 * m + (lane >> 2), ci = 8 * n + 2 * (lane & 3);
+                            atomicAdd(out + co * C + ci, acc[k][m][n][0]);
+                            atomicAdd(out + co * C + ci + 1, acc[k][m][n][1]);
+                            atomicAdd(out + (co + 8) * C + ci, acc[k][m][n][2]);
+                            atomicAdd(out + (co + 8) * C + ci + 1, acc[k][m][n][3]);
+                        }
                 }
             }
-            if (!owner) return;
-            for (int a = 0; a < 4; ++a)
-                for (int c = 0; c < 4; ++c)
-                    atomicAdd(&dW[(int64_t(tap) * cout + co0 + a) * C + ci0 + c], acc[4 * a + c]);
         }
 
         // BF16 forward weights, BF16 transposed weights (taps flipped, channels swapped) and the
@@ -828,6 +897,9 @@ namespace pcfd
         DBuf<uint8_t> mask;
         DBuf<int> batch_index;
         DBuf<float> scalars;        // [0] count, [1] loss
+        DBuf<bf16> eval_x;          // samples handed in by the host (learned_evaluate)
+        DBuf<uint8_t> eval_mask;
+        DBuf<float> eval_target;
         DBuf<int> error;
         bool harvesting = false;
         uint64_t wait_ns = kMaxWaitNs;   // limit of each tensor-core wait
@@ -928,22 +1000,17 @@ namespace pcfd
             cuda_check(cudaGetLastError(), "conv launch");
         }
 
-        template <int N> void weight_grad(System& s, ConvSource src, const bf16* G, int cout, int samples, float* dW)
+        template <int N, int COUT, int C>
+        void weight_grad(System& s, ConvSource src, const bf16* G, int samples, float* dW)
         {
-            constexpr int P = (N + 2) * (N + 2) * (N + 2), V = N * N * N;
-            const size_t smem = size_t(P) * src.channels * 2 + size_t(V) * cout * 2;
-            require(smem <= 200 * 1024, "learned: weight-gradient staging");
-            static size_t configured[3] = {0, 0, 0};
-            const int slot = N == 8 ? 0 : N == 4 ? 1 : 2;
-            if (smem > configured[slot])
-            {
-                cuda_check(cudaFuncSetAttribute(weight_grad_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)), "wgrad smem");
-                configured[slot] = smem;
-            }
-            const int entries = 27 * (cout / 4) * (src.channels / 4);
-            const int chunk = 8;
-            dim3 grid((entries + 255) / 256, (samples + chunk - 1) / chunk);
-            weight_grad_kernel<N><<<grid, 256, smem, launch_stream(s)>>>(src, G, cout, samples, chunk, dW);
+            constexpr int P = (N + 2) * (N + 2) * (N + 2), V = N * N * N, kStage = wgrad_stage<N>();
+            constexpr int smem = kStage * (P * (C + 8) + V * (COUT + 8)) * 2;
+            static_assert(smem <= 200 * 1024 && COUT % 16 == 0 && C % 16 == 0 && (kStage * V) % 16 == 0, "weight-gradient tiles");
+            require(src.channels == C, "learned: weight-gradient channels");
+            cuda_check(cudaFuncSetAttribute(weight_grad_kernel<N, COUT, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "wgrad smem");
+            // two CTAs (tap halves) per run of samples; runs of whole stages, about one wave of CTAs
+            const int runs = std::max(1, sm_count(s) / 2), chunk = (samples + runs * kStage - 1) / (runs * kStage) * kStage;
+            weight_grad_kernel<N, COUT, C><<<dim3(unsigned((samples + chunk - 1) / chunk), 2), 256, smem, launch_stream(s)>>>(src, G, samples, chunk, dW);
         }
 
         ConvSource source(const bf16* x, const bf16* w, int channels, int mode) { return ConvSource{x, w, channels, mode}; }
@@ -972,25 +1039,25 @@ namespace pcfd
             // dec0
             conv<8>(s, L, samples, 32, source(L.G4, wt(L, DEC0A), 16, SAME), nullptr, L.U0, false, true);
             conv<8>(s, L, samples, 16, source(L.G4, wt(L, DEC0B), 16, SAME), nullptr, L.S0, false, true);
-            weight_grad<8>(s, source(L.d1, nullptr, 32, UP), L.G4, 16, samples, g + tensor_offset(DEC0A));
-            weight_grad<8>(s, source(L.e0, nullptr, 16, SAME), L.G4, 16, samples, g + tensor_offset(DEC0B));
+            weight_grad<8, 16, 32>(s, source(L.d1, nullptr, 32, UP), L.G4, samples, g + tensor_offset(DEC0A));
+            weight_grad<8, 16, 16>(s, source(L.e0, nullptr, 16, SAME), L.G4, samples, g + tensor_offset(DEC0B));
             sum_children_relu_kernel<<<blocks_for(int64_t(samples) * 64 * 32), kThreads, 0, launch_stream(s)>>>(samples, 4, 32, L.U0, L.d1, L.G3);
             // dec1
             conv<4>(s, L, samples, 64, source(L.G3, wt(L, DEC1A), 32, SAME), nullptr, L.U1, false, true);
             conv<4>(s, L, samples, 32, source(L.G3, wt(L, DEC1B), 32, SAME), nullptr, L.S1, false, true);
-            weight_grad<4>(s, source(L.bt, nullptr, 64, UP), L.G3, 32, samples, g + tensor_offset(DEC1A));
-            weight_grad<4>(s, source(L.e1, nullptr, 32, SAME), L.G3, 32, samples, g + tensor_offset(DEC1B));
+            weight_grad<4, 32, 64>(s, source(L.bt, nullptr, 64, UP), L.G3, samples, g + tensor_offset(DEC1A));
+            weight_grad<4, 32, 32>(s, source(L.e1, nullptr, 32, SAME), L.G3, samples, g + tensor_offset(DEC1B));
             sum_children_relu_kernel<<<blocks_for(int64_t(samples) * 8 * 64), kThreads, 0, launch_stream(s)>>>(samples, 2, 64, L.U1, L.bt, L.G2);
             // bottleneck
             conv<2>(s, L, samples, 32, source(L.G2, wt(L, BOTT), 64, SAME), nullptr, L.P1, false, true);
-            weight_grad<2>(s, source(L.e1, nullptr, 32, POOL), L.G2, 64, samples, g + tensor_offset(BOTT));
+            weight_grad<2, 64, 32>(s, source(L.e1, nullptr, 32, POOL), L.G2, samples, g + tensor_offset(BOTT));
             combine_relu_kernel<<<blocks_for(int64_t(samples) * 64 * 32), kThreads, 0, launch_stream(s)>>>(samples, 4, 32, L.S1, L.P1, L.e1, L.G1);
             // enc1
             conv<4>(s, L, samples, 16, source(L.G1, wt(L, ENC1), 32, SAME), nullptr, L.P0, false, true);
-            weight_grad<4>(s, source(L.e0, nullptr, 16, POOL), L.G1, 32, samples, g + tensor_offset(ENC1));
+            weight_grad<4, 32, 16>(s, source(L.e0, nullptr, 16, POOL), L.G1, samples, g + tensor_offset(ENC1));
             combine_relu_kernel<<<blocks_for(int64_t(samples) * 512 * 16), kThreads, 0, launch_stream(s)>>>(samples, 8, 16, L.S0, L.P0, L.e0, L.G0);
             // enc0
-            weight_grad<8>(s, source(L.x0, nullptr, 16, SAME), L.G0, 16, samples, g + tensor_offset(ENC0));
+            weight_grad<8, 16, 16>(s, source(L.x0, nullptr, 16, SAME), L.G0, samples, g + tensor_offset(ENC0));
         }
 
         void convert(System& s, Learned& L)
@@ -1242,25 +1309,26 @@ namespace pcfd
         ensure_capacity(L, n);
         std::vector<uint16_t> hx(size_t(n) * 512);
         std::vector<uint8_t> hm(size_t(n) * 512);
-        std::vector<float> ht(target, target + size_t(n) * 512);
         for (size_t i = 0; i < hx.size(); ++i)
         {
             const bf16 b = __float2bfloat16_rn(x[2 * i]);
             std::memcpy(&hx[i], &b, 2);
             hm[i] = x[2 * i + 1] != 0 ? 1 : 0;
         }
-        DBuf<bf16> dx;
-        DBuf<uint8_t> dm;
-        DBuf<float> dt;
-        dx.alloc(hx.size(), false);
-        cuda_check(cudaMemcpy(dx.p, hx.data(), hx.size() * 2, cudaMemcpyHostToDevice), "upload inputs");
-        dm.upload(hm);
-        dt.upload(ht);
+        if (L.eval_x.n < hx.size())
+        {
+            L.eval_mask.alloc(hm.size(), false);
+            L.eval_target.alloc(hx.size(), false);
+            L.eval_x.alloc(hx.size(), false);
+        }
+        cuda_check(cudaMemcpyAsync(L.eval_x, hx.data(), hx.size() * sizeof(bf16), cudaMemcpyHostToDevice, s.stream), "upload inputs");
+        cuda_check(cudaMemcpyAsync(L.eval_mask, hm.data(), hm.size(), cudaMemcpyHostToDevice, s.stream), "upload masks");
+        cuda_check(cudaMemcpyAsync(L.eval_target, target, hx.size() * sizeof(float), cudaMemcpyHostToDevice, s.stream), "upload targets");
         std::vector<int> index(static_cast<size_t>(n));
         for (int i = 0; i < n; ++i) index[size_t(i)] = i;
         cuda_check(cudaMemcpyAsync(L.batch_index, index.data(), index.size() * sizeof(int), cudaMemcpyHostToDevice, s.stream), "indices");
         cuda_check(cudaMemsetAsync(L.scalars, 0, sizeof(float), s.stream), "zero count");
-        gather_batch_kernel<<<blocks_for(int64_t(n) * 512), kThreads, 0, launch_stream(s)>>>(L.batch_index, n, dx, dm, dt, 1.0f, L.x0,
+        gather_batch_kernel<<<blocks_for(int64_t(n) * 512), kThreads, 0, launch_stream(s)>>>(L.batch_index, n, L.eval_x, L.eval_mask, L.eval_target, 1.0f, L.x0,
                                                                                             L.target, L.mask, L.scalars);
         forward(s, L, n);
         backward(s, L, n);
