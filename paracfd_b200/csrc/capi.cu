@@ -267,9 +267,9 @@ namespace pcfd
             s.dot_partial.alloc(4096);
             s.dot_result.alloc(16);
             s.block_partial.alloc(size_t(592) * (kMaxSet + 1));
-            s.block_result.alloc(size_t(4) * (kMaxSet + 1));
+            s.block_result.alloc(size_t(6) * (kMaxSet + 1));
             cuda_check(cudaMallocHost(&s.pinned, 16 * sizeof(double)), "pinned scalars");
-            cuda_check(cudaMallocHost(&s.pinned_block, size_t(4) * (kMaxSet + 1) * sizeof(double)), "pinned block scalars");
+            cuda_check(cudaMallocHost(&s.pinned_block, size_t(6) * (kMaxSet + 1) * sizeof(double)), "pinned block scalars");
             s.dcgs_partial.alloc(size_t(592) * (2 * kMaxSet + 4));
             s.dcgs_result.alloc(size_t(kDcgsCoefficients));
             s.dcgs_total.alloc(size_t(2 * kMaxSet + 4));

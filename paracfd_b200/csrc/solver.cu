@@ -1499,6 +1499,20 @@ namespace pcfd
                 g[0] = beta;
                 vec_scaled_copy_active(s, s.gmres_v, s.defect, 1.0 / beta);
                 int used = 0;
+                // Column col + 1 needs nothing from the host's reading of column col except whether the
+                // cycle ends there.  While the residual estimate, falling as it did last, stays at least
+                // ten times the tolerance after column col, column col + 1 is enqueued before that wait,
+                // so the device does not idle for the host's round trip and launches (a column on 65 k
+                // cells: 109 -> 99 us, on 4.2 M: 611 -> 602).  A column enqueued in vain costs its device time and leaves
+                // nothing that is read again.  The columns' work and order on the stream stay the
+                // same.  Harvesting preconditioners and the learned ones count applications: no
+                // column ahead there.
+                const bool ahead = (s.preconditioner == PCFD_PRECONDITIONER_MULTIGRID || s.preconditioner == PCFD_PRECONDITIONER_JACOBI) &&
+                                   !learned_harvesting(s);
+                double estimate_now = beta, estimate_before = 10.0 * beta;   // first column: a fall by ten
+                auto stays_above = [&]() {
+                    return ahead && estimate_now * std::min(1.0, estimate_now / estimate_before) > 10.0 * tolerance * std::sqrt(rhs2);
+                };
                 if (s.delayed_orthogonalisation)
                 {
                     // Delayed CGS2: column col's single pass pair reorthogonalises V_col (projected
@@ -1546,8 +1560,7 @@ namespace pcfd
                         return std::abs(gg[cols]);
                     };
                     // Column col's work (preconditioner, operator, both passes, coefficient readback)
-                    // is enqueued as one unit, after the host has read column col - 1's coefficients
-                    // (enqueueing the next column ahead of that wait measured no gain at 16 M cells).
+                    // is enqueued as one unit.
                     const int k = s.recycle_count;
                     auto enqueue = [&](int col) {
                         double* v = s.gmres_v.p + size_t(col) * ld;
@@ -1563,8 +1576,13 @@ namespace pcfd
                         cuda_check(cudaEventRecord(s.dcgs_ready[col & 1], s.stream), "coefficient event");
                     };
                     enqueue(0);
-                    for (int col = 0; col < cycle; ++col)
+                    for (int col = 0, queued = 1; col < cycle; ++col)
                     {
+                        if (col + 1 < cycle && stays_above())
+                        {
+                            enqueue(col + 1);
+                            queued = col + 2;
+                        }
                         cuda_check(cudaEventSynchronize(s.dcgs_ready[col & 1]), "coefficient synchronize");
                         ++result.preconditioner_applications;
                         const int m = k + col;
@@ -1598,7 +1616,13 @@ namespace pcfd
                         const double estimate = least_squares(used, false);
                         if (!std::isfinite(estimate)) { --used; --result.iterations; break; }
                         if (estimate / std::sqrt(rhs2) <= tolerance || next_norm == 0) break;
-                        if (col + 1 < cycle) enqueue(col + 1);
+                        if (queued == col + 1 && col + 1 < cycle)
+                        {
+                            enqueue(col + 1);
+                            queued = col + 2;
+                        }
+                        estimate_before = estimate_now;
+                        estimate_now = estimate;
                         prev_rho = rho;
                     }
                     if (used == 0) break;
@@ -1606,25 +1630,43 @@ namespace pcfd
                 }
                 else
                 {
-                    for (int col = 0; col < cycle; ++col)
-                    {
+                    // Column col's work: CGS2 of w = A z against [C | V_0..V_col].  The matching z -= U h_C
+                    // update is deferred: its coefficients are kept per column and applied once when
+                    // the cycle's correction is formed (z only enters the solution through Z y).
+                    // Coefficients and readback alternate between two sets of three blocks.
+                    const int k = s.recycle_count;
+                    auto enqueue = [&](int col) {
                         double* v = s.gmres_v.p + size_t(col) * ld;
                         double* zc = s.gmres_z.p + size_t(col) * ld;
                         apply_preconditioner(s, v, zc);
-                        ++result.preconditioner_applications;
                         launch_apply(s, zc, s.Ad, false);
-                        // CGS2 against [C | V_0..V_col].  The matching z -= U h_C update is deferred: its
-                        // coefficients are kept per column and applied once when the cycle's
-                        // correction is formed (z only enters the solution through Z y).
-                        const int k = s.recycle_count, m = k + col + 1;
                         VecSet Q = recycle_set(s.recycle_c.p);
                         const VecSet none{int64_t(ld)};
                         for (int row = 0; row <= col; ++row) Q.push(s.gmres_v.p + size_t(row) * ld);
-                        block_dot(s, Q, s.Ad, h1);
-                        block_update(s, Q, h1, s.Ad, none, -1.0, nullptr, 2, h2);
-                        block_update(s, Q, h2, s.Ad, none, -1.0, nullptr, 1, h3);
-                        scale_by_inverse_norm(s, s.gmres_v.p + size_t(col + 1) * ld, s.Ad, h3);
-                        read_block(3);
+                        const size_t set = size_t(col & 1) * 3 * kStride;
+                        double *b1 = h1 + set, *b2 = b1 + kStride, *b3 = b2 + kStride;
+                        block_dot(s, Q, s.Ad, b1);
+                        block_update(s, Q, b1, s.Ad, none, -1.0, nullptr, 2, b2);
+                        block_update(s, Q, b2, s.Ad, none, -1.0, nullptr, 1, b3);
+                        scale_by_inverse_norm(s, s.gmres_v.p + size_t(col + 1) * ld, s.Ad, b3);
+                        cuda_check(cudaMemcpyAsync(s.pinned_block + set, b1, size_t(3) * kStride * sizeof(double), cudaMemcpyDeviceToHost,
+                                                   s.stream), "coefficient readback");
+                        cuda_check(cudaEventRecord(s.dcgs_ready[col & 1], s.stream), "coefficient event");
+                    };
+                    enqueue(0);
+                    for (int col = 0, queued = 1; col < cycle; ++col)
+                    {
+                        if (col + 1 < cycle && stays_above())
+                        {
+                            enqueue(col + 1);
+                            queued = col + 2;
+                        }
+                        cuda_check(cudaEventSynchronize(s.dcgs_ready[col & 1]), "coefficient synchronize");
+                        ++result.preconditioner_applications;
+                        const int m = k + col + 1;
+                        const double* host_h1 = s.pinned_block + size_t(col & 1) * 3 * kStride;
+                        const double* host_h2 = host_h1 + kStride;
+                        const double* host_h3 = host_h2 + kStride;
                         bool column_valid = true;
                         for (int j = 0; j < m && column_valid; ++j) column_valid = finite_value(host_h1[j]) && finite_value(host_h2[j]);
                         if (!column_valid) break;
@@ -1660,6 +1702,13 @@ namespace pcfd
                         used = col + 1;
                         ++result.iterations;
                         if (std::abs(g[col + 1]) / std::sqrt(rhs2) <= tolerance || next_norm == 0) break;
+                        if (queued == col + 1 && col + 1 < cycle)
+                        {
+                            enqueue(col + 1);
+                            queued = col + 2;
+                        }
+                        estimate_before = estimate_now;
+                        estimate_now = std::abs(g[col + 1]);
                     }
                     if (used == 0) break;
                     for (int row = used - 1; row >= 0; --row)
