@@ -9,18 +9,17 @@
 // oracle/unet.py.
 //
 // Convolutions run on the 5th-generation tensor cores: tcgen05.mma kind::f16 (BF16 operands,
-// FP32 accumulators in TMEM), M = 128 output voxels x N = Cout x K = 16 input channels per
-// instruction.  A CTA stages a group of bricks into shared memory in a zero-padded K-major
-// layout ([channel chunk of 8][padded voxel][8 x BF16]), so that the A operand of every tap
-// (dz,dy,dx) is the same layout shifted by a constant number of 16-byte rows: each tap is one
-// shared-memory descriptor, no im2col copy.  On the 8^3 level a tile is 16 padded (z,y) rows of
-// 8 voxels (stride 10 rows); on the 4^3 and 2^3 levels a tile is 128 consecutive padded
-// positions.  Rows that fall on padding are computed and discarded.
+// FP32 accumulators in TMEM), M = 128 output positions x N = 3 Cout (the three x taps) x K = 16 input
+// channels per instruction.  A CTA stages a group of bricks into shared memory in a K-major layout with
+// zero rows around every (z, y) plane ([channel chunk of 8][position][8 x BF16]), so that the A operand
+// of every (dz, dy) pair is the same layout shifted by whole rows: each pair is one shared-memory
+// descriptor, no im2col copy.  A tile is 128 consecutive positions; rows that fall on padding are
+// computed and discarded.  The epilogue adds the three x blocks across neighbouring lanes.
 //
 // Training (pcfd_learned_train): (residual, multigrid correction) brick pairs harvested from the
 // solver's own preconditioner calls, masked mean-square loss on z/s, backward pass with the
 // transposed convolutions on the same tensor-core kernel (flipped taps, transposed channels),
-// weight gradients on CUDA cores in FP32, Adam on FP32 master weights.
+// weight gradients on mma.sync tiles (BF16 operands, FP32 sums), Adam on FP32 master weights.
 #include "pcfd_internal.h"
 
 #include <cuda_bf16.h>
@@ -55,65 +54,50 @@ namespace pcfd
         constexpr uint64_t kMaxWaitNs = 2000000000ull;
 
         // ---- geometry of one level's staged group of bricks ----
-        // N: brick edge; XP: padded edge; NB: bricks per CTA; G: positions between the 8-row
-        // groups of a tile; T: tiles per group; NPOS: staged positions per channel chunk.
-        template <int N> struct Geometry;
-        template <> struct Geometry<8>
+        // NB bricks per CTA; rows (z, y) padded by one on each side, x as it is: position
+        // ((b * ROWS + (z + 1) (N + 2) + y + 1) N + x.  A tile is 128 consecutive positions (N = 8: 16 padded
+        // rows of 8, five tiles cover a brick's rows 11..90; N = 4: 32 rows of 4, one tile from row 7 covers
+        // a brick; N = 2: 64 rows of 2, a tile covers four bricks from row 5).
+        template <int N, int NB> struct Geometry
         {
-            static constexpr int XP = 10, P = 1000, NB = 2, G = 10, T = 10, NPOS = 2024;
-            // tile k of brick b starts at padded row 11 + 16 (k % 5), x = 0
-            __host__ __device__ static constexpr int tile_start(int t) { return (t / 5) * P + (11 + 16 * (t % 5)) * XP + 1; }
+            static constexpr int XP = N + 2, ROWS = XP * XP, P = ROWS * N, FIRST = XP + 1;
+            static constexpr int T = N == 8 ? 5 * NB : N == 4 ? NB : NB / 4;
+            __host__ __device__ static constexpr int tile_start(int t)
+            {
+                return N == 8 ? (t / 5) * P + (FIRST + 16 * (t % 5)) * N : N == 4 ? t * P + FIRST * N : FIRST * N + 128 * t;
+            }
+            // staged positions: the last tile plus the largest shift, in whole 8-position groups
+            static constexpr int NPOS = (tile_start(T - 1) + 128 + FIRST * N + 7) / 8 * 8;
         };
-        template <> struct Geometry<4>
-        {
-            static constexpr int XP = 6, P = 216, NB = 4, G = 8, T = 7, NPOS = 984;
-            __host__ __device__ static constexpr int tile_start(int t) { return 43 + 128 * t; }
-        };
-        template <> struct Geometry<2>
-        {
-            static constexpr int XP = 4, P = 64, NB = 16, G = 8, T = 8, NPOS = 1072;
-            __host__ __device__ static constexpr int tile_start(int t) { return 21 + 128 * t; }
-        };
-        // padded position of voxel (x,y,z) of brick b
         template <int N> __host__ __device__ constexpr int padded(int b, int x, int y, int z)
         {
-            using Gm = Geometry<N>;
-            return b * Gm::P + ((z + 1) * Gm::XP + y + 1) * Gm::XP + x + 1;
+            return (b * (N + 2) * (N + 2) + (z + 1) * (N + 2) + y + 1) * N + x;
         }
-        // M row m of tile t -> padded position
-        template <int N> __host__ __device__ constexpr int row_position(int t, int m)
-        {
-            using Gm = Geometry<N>;
-            return Gm::tile_start(t) + (m >> 3) * Gm::G + (m & 7);
-        }
-        template <int N> __host__ __device__ constexpr int tap_shift(int tap)
-        {
-            using Gm = Geometry<N>;
-            return ((tap / 9) - 1) * Gm::XP * Gm::XP + ((tap / 3) % 3 - 1) * Gm::XP + (tap % 3) - 1;
-        }
+        // shift in positions of the (dz, dy) pair zy = 3 (dz + 1) + dy + 1
+        template <int N> __host__ __device__ constexpr int row_shift(int zy) { return ((zy / 3 - 1) * (N + 2) + zy % 3 - 1) * N; }
         // compile-time proof that every descriptor stays inside the staged rows and that the
         // tiles cover every interior voxel of every brick of a group
-        template <int N> constexpr bool geometry_in_bounds()
+        template <int N, int NB> constexpr bool geometry_in_bounds()
         {
-            using Gm = Geometry<N>;
-            bool seen[Gm::NB * Gm::P] = {};
+            using Gm = Geometry<N, NB>;
+            bool seen[NB * Gm::P] = {};
             for (int t = 0; t < Gm::T; ++t)
-                for (int m = 0; m < 128; ++m)
-                {
-                    const int p = row_position<N>(t, m);
-                    if (p + tap_shift<N>(0) < 0 || p + tap_shift<N>(26) >= Gm::NPOS) return false;
-                    if (p < Gm::NB * Gm::P) seen[p] = true;
-                }
-            for (int b = 0; b < Gm::NB; ++b)
+            {
+                const int p0 = Gm::tile_start(t);
+                if (p0 + row_shift<N>(0) < 0 || p0 + 127 + row_shift<N>(8) >= Gm::NPOS) return false;
+                for (int p = p0; p < p0 + 128; ++p)
+                    if (p < NB * Gm::P) seen[p] = true;
+            }
+            for (int b = 0; b < NB; ++b)
                 for (int z = 0; z < N; ++z)
                     for (int y = 0; y < N; ++y)
                         for (int x = 0; x < N; ++x)
                             if (!seen[padded<N>(b, x, y, z)]) return false;
             return Gm::NPOS % 8 == 0;
         }
-        static_assert(geometry_in_bounds<2>(), "2^3 tiling out of bounds");
-        static_assert(geometry_in_bounds<4>(), "4^3 tiling out of bounds");
-        static_assert(geometry_in_bounds<8>(), "8^3 tiling out of bounds");
+        static_assert(geometry_in_bounds<2, 8>(), "2^3 tiling out of bounds");
+        static_assert(geometry_in_bounds<4, 4>() && geometry_in_bounds<4, 2>(), "4^3 tiling out of bounds");
+        static_assert(geometry_in_bounds<8, 1>(), "8^3 tiling out of bounds");
 
         // ---- tcgen05 / mbarrier primitives (inline PTX) ----
         __device__ inline uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -128,10 +112,10 @@ namespace pcfd
             d |= uint64_t(1) << 46;   // descriptor version (sm_100)
             return d;                 // base offset 0, swizzle none
         }
-        // kind::f16 instruction descriptor: BF16 A and B (K-major), FP32 D, M = 128, N = cout
-        __host__ __device__ constexpr uint32_t instruction_descriptor(int cout)
+        // kind::f16 instruction descriptor: BF16 A and B (K-major), FP32 D, M = 128, N = n
+        __host__ __device__ constexpr uint32_t instruction_descriptor(int n)
         {
-            return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(cout >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+            return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
         }
         __device__ inline void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate)
         {
@@ -225,6 +209,7 @@ namespace pcfd
         }
 
         // ---- convolution ----
+        constexpr int kConvThreads = 256;
         enum SourceMode { SAME = 0, POOL = 1, UP = 2 };
         struct ConvSource
         {
@@ -236,6 +221,7 @@ namespace pcfd
         {
             ConvSource src[2];
             int sources, cout, samples, relu, out_fp32;
+            int weight_slots;  // staged 16-channel weight blocks: all of the layer's, or two buffers
             void* y;           // [samples][N^3][cout], BF16 or FP32
             int* error;        // set to 1 when a barrier wait gave up
             uint64_t wait_ns;  // limit of each tensor-core wait
@@ -288,117 +274,139 @@ namespace pcfd
             asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
         }
 
-        // One CTA of 128 threads per group of Geometry<N>::NB bricks (persistent over groups).
-        // Shared memory: A [2][NPOS][16 B] | B [27][2][cout][16 B] | barrier | TMEM address.
-        template <int N>
-        __global__ void __launch_bounds__(128) conv_kernel(ConvParams p)
+        // One CTA of 256 threads per group of NB bricks (persistent over groups).  The three x taps of a
+        // (dz, dy) pair run as ONE MMA of N = 3 cout columns against the same A tile: column block dx of
+        // row x holds W[dz, dy, dx] in[z + dz, y + dy, x], and the epilogue adds the blocks of x - 1, x and
+        // x + 1, neighbouring lanes of a warp.  An MMA's time is its shared-memory reads (128 B per
+        // clock: 4 KiB of A, 32 B per column of B), so 9 MMAs of 48 columns (43 clocks) replace 27 of 16 (36);
+        // x needs no padding, and at the 4^3 level a tile holds one brick's rows at half instead of a
+        // quarter of its lanes.
+        // Two buffers of A (and of B, unless the layer's weights fit whole): the next 16 channels, also of
+        // the next group, are staged while the MMAs run.
+        // Shared memory: A [2][2][NPOS][16 B] | B [slots][9][2][3 cout][16 B] | barriers | TMEM address.
+        template <int N, int NB>
+        __global__ void __launch_bounds__(kConvThreads) conv_kernel(ConvParams p)
         {
-            using Gm = Geometry<N>;
+            using Gm = Geometry<N, NB>;
             extern __shared__ __align__(128) uint8_t smem[];
             uint4* A = reinterpret_cast<uint4*>(smem);
-            const int cout = p.cout;
-            uint4* Bw = A + 2 * Gm::NPOS;
-            uint64_t* bar = reinterpret_cast<uint64_t*>(Bw + 27 * 2 * cout);
+            const int cout = p.cout, n3 = 3 * cout, b_size = 9 * 2 * n3;
+            uint4* Bw = A + 4 * Gm::NPOS;
+            uint64_t* bar = reinterpret_cast<uint64_t*>(Bw + p.weight_slots * b_size);
             uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
             uint64_t* idle = bar + 2;      // initialised, never arrived on
             __shared__ int failed;
             const int tid = threadIdx.x, warp = tid >> 5;
-            const uint32_t cols = tmem_columns(Gm::T * cout);
+            const uint32_t cols = tmem_columns(Gm::T * n3);
 
-            for (int i = tid; i < 2 * Gm::NPOS; i += 128) A[i] = make_uint4(0, 0, 0, 0);
+            for (int i = tid; i < 4 * Gm::NPOS; i += kConvThreads) A[i] = make_uint4(0, 0, 0, 0);
             if (tid == 0) { barrier_init(bar); barrier_init(idle); failed = 0; }
             if (warp == 0) tmem_alloc(tslot, cols);
             fence_before_sync();
             __syncthreads();
             fence_after_sync();
             const uint32_t tmem = *tslot;
-            const uint32_t a_base = smem_u32(A), b_base = smem_u32(Bw);
-            const uint32_t idesc = instruction_descriptor(cout);
+            const uint32_t idesc = instruction_descriptor(n3);
             uint32_t phase = 0;
-            const int groups = (p.samples + Gm::NB - 1) / Gm::NB;
+            const int groups = (p.samples + NB - 1) / NB;
             constexpr int V = N * N * N;
+            int chunks = 0;                // of 16 channels, over both sources
+            for (int si = 0; si < p.sources; ++si) chunks += p.src[si].channels / 16;
+            const bool resident = p.weight_slots >= chunks;
 
+            // stages 16 channels of the group's bricks and the matching weights: copies straight to shared
+            // memory (cp.async) for plain and upsampled sources, a register average for pooled ones
+            auto stage = [&](int group, int chunk, int slot, bool weights) {
+                int si = 0, c0 = 16 * chunk;
+                if (c0 >= p.src[0].channels) { si = 1; c0 -= p.src[0].channels; }
+                const ConvSource& s = p.src[si];
+                const int b0 = group * NB, items = min(NB, p.samples - b0) * V * 2;
+                uint4* a = A + slot * 2 * Gm::NPOS;
+                for (int i = tid; i < items; i += kConvThreads)
+                {
+                    const int half = i & 1, v = (i >> 1) % V, b = (i >> 1) / V;
+                    const int x = v % N, y = (v / N) % N, z = v / (N * N);
+                    uint4* to = &a[half * Gm::NPOS + padded<N>(b, x, y, z)];
+                    if (s.mode != POOL) cp_async16(to, source_address<N>(s, b0 + b, x, y, z, c0 + 8 * half));
+                    else *to = load_source<N>(s, b0 + b, x, y, z, c0 + 8 * half);
+                }
+                if (!weights) return;
+                uint4* w = Bw + (resident ? chunk : slot) * b_size;
+                for (int i = tid; i < b_size; i += kConvThreads)
+                {
+                    const int n = i % n3, half = (i / n3) & 1, zy = i / (2 * n3);
+                    cp_async16(&w[i], s.w + (int64_t(zy) * n3 + n) * s.channels + c0 + 8 * half);
+                }
+            };
+
+            int slot = 0;
+            bool loaded = false;            // resident weights staged
+            if (int(blockIdx.x) < groups)
+            {
+                stage(blockIdx.x, 0, 0, true);
+                cp_async_wait_all();
+                fence_async_shared();
+                __syncthreads();
+            }
             for (int group = blockIdx.x; group < groups; group += gridDim.x)
             {
-                const int b0 = group * Gm::NB, nb = min(Gm::NB, p.samples - b0);
-                bool first = true;
-                for (int si = 0; si < p.sources; ++si)
+                const int b0 = group * NB, nb = min(NB, p.samples - b0);
+                for (int chunk = 0; chunk < chunks; ++chunk, slot ^= 1)
                 {
-                    const ConvSource& s = p.src[si];
-                    for (int c0 = 0; c0 < s.channels; c0 += 16)
+                    if (tid == 0)
                     {
-                        // stage 16 channels of the group's bricks and the matching weights: copies
-                        // straight to shared memory (cp.async) for plain and upsampled sources, a
-                        // register average for pooled ones (two voxels in flight per thread)
-                        const int items = nb * V * 2;
-                        if (s.mode != POOL)
-                        {
-                            for (int i = tid; i < items; i += 128)
+                        fence_after_sync();
+                        const uint32_t a_base = smem_u32(A + slot * 2 * Gm::NPOS), b_base = smem_u32(Bw + (resident ? chunk : slot) * b_size);
+                        for (int t = 0; t < Gm::T; ++t)
+                            for (int zy = 0; zy < 9; ++zy)
                             {
-                                const int half = i & 1, v = (i >> 1) % V, b = (i >> 1) / V;
-                                const int x = v % N, y = (v / N) % N, z = v / (N * N);
-                                cp_async16(&A[half * Gm::NPOS + padded<N>(b, x, y, z)], source_address<N>(s, b0 + b, x, y, z, c0 + 8 * half));
+                                const uint64_t a = smem_descriptor(a_base + uint32_t(Gm::tile_start(t) + row_shift<N>(zy)) * 16u,
+                                                                   uint32_t(Gm::NPOS) * 16u, 128u);
+                                const uint64_t b = smem_descriptor(b_base + uint32_t(zy * 2 * n3) * 16u, uint32_t(n3) * 16u, 128u);
+                                mma_bf16(tmem + uint32_t(t * n3), a, b, idesc, (chunk == 0 && zy == 0) ? 0u : 1u);
                             }
-                        }
-                        else
-                        {
-                            for (int i = tid; i < items; i += 256)
-                            {
-                                const int j = i + 128;
-                                uint4 u0, u1 = make_uint4(0, 0, 0, 0);
-                                const int h0 = i & 1, v0 = (i >> 1) % V, bb0 = (i >> 1) / V;
-                                u0 = load_source<N>(s, b0 + bb0, v0 % N, (v0 / N) % N, v0 / (N * N), c0 + 8 * h0);
-                                const int h1 = j & 1, v1 = (j >> 1) % V, bb1 = (j >> 1) / V;
-                                if (j < items) u1 = load_source<N>(s, b0 + bb1, v1 % N, (v1 / N) % N, v1 / (N * N), c0 + 8 * h1);
-                                A[h0 * Gm::NPOS + padded<N>(bb0, v0 % N, (v0 / N) % N, v0 / (N * N))] = u0;
-                                if (j < items) A[h1 * Gm::NPOS + padded<N>(bb1, v1 % N, (v1 / N) % N, v1 / (N * N))] = u1;
-                            }
-                        }
-                        for (int i = tid; i < 27 * 2 * cout; i += 128)
-                        {
-                            const int co = i % cout, half = (i / cout) & 1, tap = i / (2 * cout);
-                            cp_async16(&Bw[i], s.w + (int64_t(tap) * cout + co) * s.channels + c0 + 8 * half);
-                        }
-                        cp_async_wait_all();
-                        fence_async_shared();
-                        __syncthreads();
-                        if (tid == 0)
-                        {
-                            fence_after_sync();
-                            for (int t = 0; t < Gm::T; ++t)
-                                for (int tap = 0; tap < 27; ++tap)
-                                {
-                                    const uint64_t a = smem_descriptor(a_base + uint32_t(Gm::tile_start(t) + tap_shift<N>(tap)) * 16u,
-                                                                       uint32_t(Gm::NPOS) * 16u, uint32_t(Gm::G) * 16u);
-                                    const uint64_t b = smem_descriptor(b_base + uint32_t(tap) * 2u * uint32_t(cout) * 16u, uint32_t(cout) * 16u, 128u);
-                                    mma_bf16(tmem + uint32_t(t * cout), a, b, idesc, (first && tap == 0) ? 0u : 1u);
-                                }
-                            mma_commit(bar);
-                        }
-                        first = false;
-                        const bool done = p.idle_wait ? barrier_wait(idle, 0, p.wait_ns) : barrier_wait(bar, phase, p.wait_ns);
-                        if (!done) failed = 1;
-                        phase ^= 1;
-                        __syncthreads();
-                        if (failed) break;
+                        mma_commit(bar);
                     }
+                    // the next chunk goes into the other buffer, whose MMAs have been waited for
+                    const bool next_group = chunk + 1 == chunks;
+                    const int after = next_group ? group + int(gridDim.x) : group;
+                    if (after < groups) stage(after, next_group ? 0 : chunk + 1, slot ^ 1, !(resident && (loaded || next_group)));
+                    const bool done = p.idle_wait ? barrier_wait(idle, 0, p.wait_ns) : barrier_wait(bar, phase, p.wait_ns);
+                    if (!done) failed = 1;
+                    phase ^= 1;
+                    cp_async_wait_all();
+                    fence_async_shared();
+                    __syncthreads();
                     if (failed) break;
                 }
+                loaded = true;
                 if (failed) break;
-                // epilogue: TMEM lane = tile row; warp w reads lanes 32w..32w+31
+                // epilogue: TMEM lane = tile row; warps w and w + 4 read lanes 32 (w % 4) .. + 31, alternate tiles
                 fence_after_sync();
-                for (int t = 0; t < Gm::T; ++t)
+                const int m = 32 * (warp & 3) + (tid & 31), x = m % N;
+                for (int t = warp >> 2; t < Gm::T; t += 2)
                 {
-                    const int m = 32 * warp + (tid & 31);
-                    const int pos = row_position<N>(t, m);
-                    const int b = pos / Gm::P, rem = pos % Gm::P;
-                    const int zp = rem / (Gm::XP * Gm::XP), yp = (rem / Gm::XP) % Gm::XP, xp = rem % Gm::XP;
-                    const bool valid = b < nb && zp >= 1 && zp <= N && yp >= 1 && yp <= N && xp >= 1 && xp <= N;
-                    const int64_t voxel = (int64_t(b0 + b) * V + ((zp - 1) * N + (yp - 1)) * N + (xp - 1));
+                    const int pos = Gm::tile_start(t) + m;
+                    const int b = pos / Gm::P, row = (pos % Gm::P) / N, zp = row / Gm::XP, yp = row % Gm::XP;
+                    const bool valid = b < nb && zp >= 1 && zp <= N && yp >= 1 && yp <= N;
+                    const int64_t voxel = (int64_t(b0 + b) * V + ((zp - 1) * N + (yp - 1)) * N + x);
                     for (int c = 0; c < cout; c += 16)
                     {
-                        float v[16];
-                        tmem_load16(tmem + (uint32_t(32 * warp) << 16) + uint32_t(t * cout + c), v);
+                        const uint32_t at = tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(t * n3 + c);
+                        float v[16], w[16];
+                        tmem_load16(at + uint32_t(cout), v);              // dx = 0
+                        tmem_load16(at, w);                               // dx = -1, from x - 1
+                        for (int i = 0; i < 16; ++i)
+                        {
+                            const float left = __shfl_up_sync(0xffffffffu, w[i], 1);
+                            v[i] += x > 0 ? left : 0.0f;
+                        }
+                        tmem_load16(at + uint32_t(2 * cout), w);          // dx = +1, from x + 1
+                        for (int i = 0; i < 16; ++i)
+                        {
+                            const float right = __shfl_down_sync(0xffffffffu, w[i], 1);
+                            v[i] += x < N - 1 ? right : 0.0f;
+                        }
                         if (!valid) continue;
                         if (p.relu)
                             for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
@@ -430,11 +438,13 @@ namespace pcfd
             if (warp == 0) tmem_dealloc(tmem, cols);
         }
 
-        template <int N> size_t conv_smem(int cout)
+        // weights kept whole up to 44 KiB, else two buffers
+        inline int weight_slots(int chunks, int cout) { return chunks * 9 * 2 * 3 * cout * 16 <= 44 * 1024 ? std::max(1, chunks) : 2; }
+        template <int N, int NB> size_t conv_smem(int cout, int slots)
         {
-            const size_t bytes = size_t(2) * Geometry<N>::NPOS * 16 + size_t(27) * 2 * cout * 16 + 32;
+            const size_t bytes = size_t(4) * Geometry<N, NB>::NPOS * 16 + size_t(slots) * 9 * 2 * 3 * cout * 16 + 32;
             // co-resident CTAs must fit their TMEM allocations into the SM's 512 columns
-            const int cols = tmem_columns(Geometry<N>::T * cout);
+            const int cols = tmem_columns(Geometry<N, NB>::T * 3 * cout);
             const size_t floor_bytes = cols == 512 ? 116 * 1024 : cols == 256 ? 80 * 1024 : cols == 128 ? 48 * 1024 : 0;
             return std::max(bytes, floor_bytes);
         }
@@ -965,6 +975,19 @@ namespace pcfd
             return count;
         }
 
+        template <int N, int NB>
+        void launch_conv(System& s, ConvParams p, int chunks)
+        {
+            p.weight_slots = weight_slots(chunks, p.cout);
+            const size_t smem = conv_smem<N, NB>(p.cout, p.weight_slots);
+            require(Geometry<N, NB>::T * 3 * p.cout <= 512 && smem <= 226 * 1024, "learned: output channels");
+            // the largest request of any layer, so that one layer never lowers another's
+            cuda_check(cudaFuncSetAttribute(conv_kernel<N, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024), "conv smem");
+            const int groups = (p.samples + NB - 1) / NB;
+            const int per_sm = smem > 114 * 1024 ? 1 : smem > 76 * 1024 ? 2 : 3;
+            conv_kernel<N, NB><<<std::min(groups, sm_count(s) * per_sm), kConvThreads, smem, launch_stream(s)>>>(p);
+            cuda_check(cudaGetLastError(), "conv launch");
+        }
         template <int N>
         void conv(System& s, Learned& L, int samples, int cout, ConvSource a, const ConvSource* b, void* y, bool relu, bool fp32)
         {
@@ -973,9 +996,13 @@ namespace pcfd
             p.src[0] = a;
             p.sources = 1;
             if (b) { p.src[1] = *b; p.sources = 2; }
+            int chunks = 0;
             for (int k = 0; k < p.sources; ++k)
+            {
                 require(p.src[k].channels % 16 == 0 && p.src[k].channels <= 64, "learned: channel count");
-            require(cout % 16 == 0 && cout <= 64 && Geometry<N>::T * cout <= 512, "learned: output channels");
+                chunks += p.src[k].channels / 16;
+            }
+            require(cout % 16 == 0 && cout <= 64, "learned: output channels");
             p.cout = cout;
             p.samples = samples;
             p.relu = relu;
@@ -985,19 +1012,15 @@ namespace pcfd
             p.wait_ns = L.wait_ns;
             p.idle_wait = L.idle_wait_once ? 1 : 0;
             L.idle_wait_once = false;
-            const size_t smem = conv_smem<N>(cout);
-            static size_t configured[3] = {0, 0, 0};
-            const int slot = N == 8 ? 0 : N == 4 ? 1 : 2;
-            if (smem > configured[slot])
+            // bricks per CTA: as many tiles as the 512 TMEM columns hold, but one at the 8^3 level, where two
+            // CTAs per SM then overlap their staging, MMAs and epilogues
+            if constexpr (N == 8) launch_conv<8, 1>(s, p, chunks);
+            else if constexpr (N == 4)
             {
-                cuda_check(cudaFuncSetAttribute(conv_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)), "conv smem");
-                configured[slot] = smem;
+                if (cout <= 32) launch_conv<4, 4>(s, p, chunks);
+                else launch_conv<4, 2>(s, p, chunks);
             }
-            const int groups = (samples + Geometry<N>::NB - 1) / Geometry<N>::NB;
-            const int per_sm = smem > 114 * 1024 ? 1 : smem > 76 * 1024 ? 2 : 3;
-            const int grid = std::min(groups, sm_count(s) * per_sm);
-            conv_kernel<N><<<grid, 128, smem, launch_stream(s)>>>(p);
-            cuda_check(cudaGetLastError(), "conv launch");
+            else launch_conv<2, 8>(s, p, chunks);
         }
 
         template <int N, int COUT, int C>
