@@ -189,27 +189,25 @@ namespace pcfd
             if (kMode != 0) block_store<V>(acc, kMode == 1 ? 0 : count, partial);
         }
 
-        // out[j] = sum over blocks of partial[b * kStride + j], j <= count (fixed order).
-        __global__ void __launch_bounds__(256) block_final_kernel(const double* __restrict__ partial, int blocks, int count,
-                                                                  double* __restrict__ out)
+        // out[j] = sum over blocks of partial[b * kStride + j], one CTA per sum j: thread partials over
+        // b = t, t + 256, ..., a warp tree, then the 8 warps in order.  In one CTA all the sums' loads
+        // queued behind each other: 12.8 us on average over the columns of a cycle.
+        __global__ void __launch_bounds__(256) block_final_kernel(const double* __restrict__ partial, int blocks, double* __restrict__ out)
         {
-            // thread partials over b = t, t + 256, ..., a warp tree, then the 8 warps in order; no
-            // barrier inside the loop over j, so the sums' loads overlap
-            __shared__ double shared[8][kStride];
-#pragma unroll 4
-            for (int j = 0; j <= count; ++j)
-            {
-                double v = 0.0;
-                for (int b = threadIdx.x; b < blocks; b += blockDim.x) v += partial[int64_t(b) * kStride + j];
-                v = warp_sum(v);
-                if ((threadIdx.x & 31) == 0) shared[threadIdx.x >> 5][j] = v;
-            }
+            chain_wait();
+            chain_release();
+            __shared__ double shared[8];
+            const int j = blockIdx.x;
+            double v = 0.0;
+            for (int b = threadIdx.x; b < blocks; b += blockDim.x) v += partial[int64_t(b) * kStride + j];
+            v = warp_sum(v);
+            if ((threadIdx.x & 31) == 0) shared[threadIdx.x >> 5] = v;
             __syncthreads();
-            if (threadIdx.x <= count)
+            if (threadIdx.x == 0)
             {
                 double t = 0.0;
-                for (int w = 0; w < 8; ++w) t += shared[w][threadIdx.x];
-                out[threadIdx.x] = t;
+                for (int w = 0; w < 8; ++w) t += shared[w];
+                out[j] = t;
             }
         }
 
@@ -254,93 +252,81 @@ namespace pcfd
         // Pass 1 for Q = [C | V_0..V_{j-1}] (final), v = V_j (projected once) and w = A z_j:
         // s = Q^T v, t = Q^T w, v.v, v.w, w.w -> partial[block][2 * kMaxSet + 3].
         constexpr int kDcgsStride = 2 * kMaxSet + 4;
-        // Warp w of a CTA takes basis vectors [V w, V w + V), V = ceil(m / 8), and its 32 lanes walk
-        // consecutive element pairs, so every load of a warp reads 512 contiguous bytes of one
-        // vector.  Every warp reads v and w as well (mostly from L1); warp 0 also sums v.v, v.w and
-        // w.w.  A lane loads kGroup sub-blocks of pairs before it sums, to keep enough bytes in
-        // flight with few vectors per warp.  Each sum is per lane over the CTA's items, then a warp
-        // reduction; partial[block][j] holds the owning warp's sum.
-        template <int V>
-        __host__ __device__ constexpr int dcgs_group() { return V <= 2 ? 2 : 1; }
-        template <int V>
+        // The CTA's eight warps form GROUPS groups; group g takes basis vectors [V g, V g + V) and its
+        // 8 / GROUPS warps share the element pairs, a warp reading 512 contiguous bytes of one vector
+        // per load.  With up to four vectors there is one group: every element is read once and all
+        // warps work (a warp per vector left 8 - m of them idle and read v and w m times: 309 us
+        // on average for m <= 8 on 19 M entries, now 192: 80 for m <= 2, 137 for 3 and 4, 288 for 5 to 8).
+        // More vectors need more groups for the registers: 2 V running sums and V loads per lane;
+        // v and w are then read once per group.  Measured at the same size: m 5 to 8 as one group of
+        // eight 299, 9 to 13 as two of eight 372 and as four of four 582 us.  Group 0 also sums v.v, v.w
+        // and w.w.  Each sum is per lane over the CTA's items, then a warp reduction, then the
+        // group's warps in order; partial[block][j] holds the CTA's sum.
+        template <int V, int GROUPS>
         __global__ void __launch_bounds__(kThreadsBlock) dcgs_dot_kernel(VecSet Q, const double* __restrict__ vv,
             const double* __restrict__ w, const uint8_t* __restrict__ active, Sweep range, double* __restrict__ partial)
         {
-            __shared__ double shared[kDcgsStride];
+            constexpr int kWarps = kThreadsBlock / 32, kShare = kWarps / GROUPS;     // warps per group
+            constexpr int kSubBlocks = 512 / 64;       // an item is 512 entries = 8 sub-blocks of 32 pairs
+            __shared__ double shared[kWarps][2 * V + 3];
             double as[V], at[V], vv2 = 0.0, vw = 0.0, ww = 0.0;
 #pragma unroll
             for (int u = 0; u < V; ++u) { as[u] = 0.0; at[u] = 0.0; }
             const int count = Q.size();
             const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            const int first = V * warp;
-            const bool norms = warp == 0;
-            constexpr int kGroup = dcgs_group<V>();
-            constexpr int kSubBlocks = 512 / 64;       // an item is 512 entries = 8 sub-blocks of 32 pairs
-            if (first < count || norms)
-                for (int64_t item = blockIdx.x; item < range.items; item += gridDim.x)
-                {
-                    const int64_t base = range.base(item);
+            const int first = V * (warp / kShare), share = warp % kShare;
+            const bool norms = warp < kShare;
+            for (int64_t item = blockIdx.x; item < range.items; item += gridDim.x)
+            {
+                const int64_t base = range.base(item);
 #pragma unroll 1
-                    for (int sub0 = 0; sub0 < kSubBlocks; sub0 += kGroup)
+                for (int sub = share; sub < kSubBlocks; sub += kShare)
+                {
+                    const int64_t e = base + 2 * (32 * sub + lane);
+                    const bool valid = e < range.padded;
+                    const int64_t q = valid ? e >> 1 : 0;
+                    const uchar2 a = valid ? reinterpret_cast<const uchar2*>(active)[q] : make_uchar2(0, 0);
+                    const double2 v0 = valid ? reinterpret_cast<const double2*>(vv)[q] : make_double2(0.0, 0.0);
+                    const double2 w0 = valid ? reinterpret_cast<const double2*>(w)[q] : make_double2(0.0, 0.0);
+                    double2 b[V];
+#pragma unroll
+                    for (int u = 0; u < V; ++u)
+                        b[u] = valid && first + u < count ? reinterpret_cast<const double2*>(Q.vec(first + u))[q] : make_double2(0.0, 0.0);
+                    const double vx = a.x ? v0.x : 0.0, vy = a.y ? v0.y : 0.0, wx = a.x ? w0.x : 0.0, wy = a.y ? w0.y : 0.0;
+#pragma unroll
+                    for (int u = 0; u < V; ++u)
                     {
-                        uchar2 a[kGroup];
-                        double2 v0[kGroup], w0[kGroup], b[kGroup][V];
-#pragma unroll
-                        for (int g = 0; g < kGroup; ++g)
-                        {
-                            const int64_t e = base + 2 * (32 * (sub0 + g) + lane);
-                            const bool valid = e < range.padded;
-                            const int64_t q = valid ? e >> 1 : 0;
-                            a[g] = valid ? reinterpret_cast<const uchar2*>(active)[q] : make_uchar2(0, 0);
-                            v0[g] = valid ? reinterpret_cast<const double2*>(vv)[q] : make_double2(0.0, 0.0);
-                            w0[g] = valid ? reinterpret_cast<const double2*>(w)[q] : make_double2(0.0, 0.0);
-#pragma unroll
-                            for (int u = 0; u < V; ++u)
-                                b[g][u] = valid && first + u < count ? reinterpret_cast<const double2*>(Q.vec(first + u))[q]
-                                                                     : make_double2(0.0, 0.0);
-                        }
-#pragma unroll
-                        for (int g = 0; g < kGroup; ++g)
-                        {
-#pragma unroll
-                            for (int u = 0; u < V; ++u)
-                            {
-                                as[u] += (a[g].x ? b[g][u].x * v0[g].x : 0.0) + (a[g].y ? b[g][u].y * v0[g].y : 0.0);
-                                at[u] += (a[g].x ? b[g][u].x * w0[g].x : 0.0) + (a[g].y ? b[g][u].y * w0[g].y : 0.0);
-                            }
-                            if (norms)
-                            {
-                                vv2 += (a[g].x ? v0[g].x * v0[g].x : 0.0) + (a[g].y ? v0[g].y * v0[g].y : 0.0);
-                                vw += (a[g].x ? v0[g].x * w0[g].x : 0.0) + (a[g].y ? v0[g].y * w0[g].y : 0.0);
-                                ww += (a[g].x ? w0[g].x * w0[g].x : 0.0) + (a[g].y ? w0[g].y * w0[g].y : 0.0);
-                            }
-                        }
+                        as[u] += b[u].x * vx + b[u].y * vy;
+                        at[u] += b[u].x * wx + b[u].y * wy;
+                    }
+                    if (norms)
+                    {
+                        vv2 += vx * vx + vy * vy;
+                        vw += vx * wx + vy * wy;
+                        ww += wx * wx + wy * wy;
                     }
                 }
-            for (int j = threadIdx.x; j < kDcgsStride; j += blockDim.x) shared[j] = 0.0;
-            __syncthreads();
+            }
 #pragma unroll
             for (int u = 0; u < V; ++u)
             {
                 const double x = warp_sum(as[u]), y = warp_sum(at[u]);
-                if (lane == 0 && first + u < count)
-                {
-                    shared[first + u] = x;
-                    shared[kMaxSet + first + u] = y;
-                }
+                if (lane == 0) { shared[warp][u] = x; shared[warp][V + u] = y; }
             }
-            if (norms)
-            {
-                const double a1 = warp_sum(vv2), a2 = warp_sum(vw), a3 = warp_sum(ww);
-                if (lane == 0)
-                {
-                    shared[2 * kMaxSet] = a1;
-                    shared[2 * kMaxSet + 1] = a2;
-                    shared[2 * kMaxSet + 2] = a3;
-                }
-            }
+            const double a1 = warp_sum(vv2), a2 = warp_sum(vw), a3 = warp_sum(ww);
+            if (lane == 0) { shared[warp][2 * V] = a1; shared[warp][2 * V + 1] = a2; shared[warp][2 * V + 2] = a3; }
             __syncthreads();
-            for (int j = threadIdx.x; j < kDcgsStride - 1; j += blockDim.x) partial[int64_t(blockIdx.x) * kDcgsStride + j] = shared[j];
+            // partial[j]: [0, kMaxSet) s, [kMaxSet, 2 kMaxSet) t, then the three norms
+            for (int j = threadIdx.x; j < kDcgsStride - 1; j += blockDim.x)
+            {
+                const bool norm = j >= 2 * kMaxSet;
+                const int vector = norm ? 0 : j % kMaxSet, group = vector / V;
+                const int slot = norm ? 2 * V + j - 2 * kMaxSet : (j < kMaxSet ? 0 : V) + vector % V;
+                double t = 0.0;
+                if (group < GROUPS)
+                    for (int k = 0; k < kShare; ++k) t += shared[group * kShare + k][slot];
+                partial[int64_t(blockIdx.x) * kDcgsStride + j] = t;
+            }
         }
 
         // Sums the pass-1 partials (fixed order) and forms the update coefficients:
@@ -411,7 +397,7 @@ namespace pcfd
         // One element pair per thread; the thread walks the basis vectors in order (j = 0, 1, ...)
         // in chunks of eight loads in flight, so each warp reads 512 contiguous bytes of every
         // vector and no sum crosses lanes.  (The dot pass cannot do the same: 2m + 3 running sums
-        // per thread would not fit its registers, so it splits the vectors across warps instead.)
+        // per thread do not fit its registers past m = 8, so it splits the vectors across warps there.)
         constexpr int kUpdateChunk = 8;
         __global__ void __launch_bounds__(kThreadsBlock) dcgs_update_kernel(VecSet Q, const double* __restrict__ coefficient,
             double* __restrict__ vv, const double* __restrict__ w, double* __restrict__ next, const uint8_t* __restrict__ active, Sweep range)
@@ -531,7 +517,8 @@ namespace pcfd
         modes(block_kernel<1, 0>, block_kernel<2, 0>, block_kernel<4, 0>, block_kernel<8, 0>);
         modes(block_kernel<1, 1>, block_kernel<2, 1>, block_kernel<4, 1>, block_kernel<8, 1>);
         modes(block_kernel<1, 2>, block_kernel<2, 2>, block_kernel<4, 2>, block_kernel<8, 2>);
-        modes(dcgs_dot_kernel<1>, dcgs_dot_kernel<2>, dcgs_dot_kernel<3>, dcgs_dot_kernel<4>);
+        modes(dcgs_dot_kernel<2, 1>, dcgs_dot_kernel<4, 1>, dcgs_dot_kernel<4, 2>, dcgs_dot_kernel<8, 2>);
+        block_grid(dcgs_dot_kernel<8, 4>);
         block_grid(dcgs_update_kernel);
     }
 
@@ -542,7 +529,7 @@ namespace pcfd
         require_aligned(Q, "block dot: vector not 16-byte aligned");
         const VecSet none(Q.stride);
         const int grid = launch_block<-1>(s, Q, nullptr, const_cast<double*>(w), none, 0.0, nullptr);
-        block_final_kernel<<<1, 256, 0, launch_stream(s)>>>(s.block_partial, grid, Q.size(), out);
+        launch_chained(s, block_final_kernel, unsigned(Q.size() + 1), 256u, s.block_partial, grid, out);
     }
 
     void block_update(System& s, const VecSet& Q, const double* h, double* w, const VecSet& U, double sign, double* y, int mode,
@@ -557,7 +544,7 @@ namespace pcfd
         else if (mode == 1) grid = launch_block<1>(s, Q, h, w, U, sign, y);
         else grid = launch_block<2>(s, Q, h, w, U, sign, y);
         if (mode >= 1)
-            block_final_kernel<<<1, 256, 0, launch_stream(s)>>>(s.block_partial, grid, mode == 2 ? Q.size() : 0, out);
+            launch_chained(s, block_final_kernel, unsigned((mode == 2 ? Q.size() : 0) + 1), 256u, s.block_partial, grid, out);
     }
 
     void dcgs_pass(System& s, const VecSet& Q, double* v, const double* w, double* next, double* coefficient)
@@ -572,11 +559,12 @@ namespace pcfd
             grid = block_grid(kernel);
             kernel<<<grid, kThreadsBlock, 0, launch_stream(s)>>>(Q, v, w, s.active, range, s.dcgs_partial);
         };
-        // V = ceil(m / 8) basis vectors per warp (kMaxSet = 32)
-        if (m <= 8) dot(dcgs_dot_kernel<1>);
-        else if (m <= 16) dot(dcgs_dot_kernel<2>);
-        else if (m <= 24) dot(dcgs_dot_kernel<3>);
-        else dot(dcgs_dot_kernel<4>);
+        // the fewest running sums that hold the m vectors (kMaxSet = 32)
+        if (m <= 2) dot(dcgs_dot_kernel<2, 1>);
+        else if (m <= 4) dot(dcgs_dot_kernel<4, 1>);
+        else if (m <= 8) dot(dcgs_dot_kernel<4, 2>);
+        else if (m <= 16) dot(dcgs_dot_kernel<8, 2>);
+        else dot(dcgs_dot_kernel<8, 4>);
         dcgs_final_kernel<<<2 * kMaxSet + 3, 256, 0, launch_stream(s)>>>(s.dcgs_partial, grid, m, s.dcgs_total, s.dcgs_ticket,
                                                                        coefficient);
         dcgs_update_kernel<<<block_grid(dcgs_update_kernel), kThreadsBlock, 0, launch_stream(s)>>>(Q, coefficient, v, w, next, s.active,
