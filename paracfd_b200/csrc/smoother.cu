@@ -5,7 +5,8 @@
 // the level-0 aggregates and prolongs the coarse correction back: ~10 full passes over the FP64
 // vectors plus a serial per-aggregate gather.  Here every fine-level stage is one brick-tiled
 // launch that reads z (tile + halo staged in shared memory), r and one code byte per DOF:
-//   sweep      z_new = z + w (r - A_struct z) / D          (ping-pong buffers)
+//   sweep      z_new = z + w (r - A_struct z) / D          (ping-pong buffers; on small grids the first
+//              sweep from zero, z = w r / D, is formed in the second's tile)
 //   residual   per-brick partial sums of r - A_struct z for each level-0 cell the brick covers
 //   prolong    the coarse correction is added while the tile is staged (z + e[aggregate])
 // The code byte holds the six open-face bits (both cells active and the face not cut), the
@@ -70,10 +71,27 @@ namespace pcfd
             return b0 + ((k >> l) << 6) + ((j >> l) << 3) + (i >> l);
         }
 
-        // Structured 7-point row of cell s of the tile (order -x,+x,-y,+y,-z,+z, then outlet);
-        // identical arithmetic to the unfused operator kernel.
-        template <class T>
-        __device__ inline T structured_row(const T* tile, int s, uint8_t code, T h)
+        template <class T> struct PairOf;
+        template <> struct PairOf<float> { using type = float2; };
+        template <> struct PairOf<double> { using type = double2; };
+        template <class T> using Pair = typename PairOf<T>::type;
+        template <class T> __device__ inline Pair<T> load_pair(const T* p) { return *reinterpret_cast<const Pair<T>*>(p); }
+
+        // Structured 7-point row (order -x,+x,-y,+y,-z,+z); the outlet term follows.  Identical arithmetic to
+        // the unfused operator kernel.
+        template <class T> __device__ inline T structured_row(T pa, T xm, T xp, T ym, T yp, T zm, T zp, uint8_t code, T h)
+        {
+            T Az = T(0);
+            if (code & 1) Az += h * (pa - xm);
+            if (code & 2) Az += h * (pa - xp);
+            if (code & 4) Az += h * (pa - ym);
+            if (code & 8) Az += h * (pa - yp);
+            if (code & 16) Az += h * (pa - zm);
+            if (code & 32) Az += h * (pa - zp);
+            return Az;
+        }
+        // The row of cell s of the tile, outlet included.
+        template <class T> __device__ inline T structured_cell(const T* tile, int s, uint8_t code, T h)
         {
             const T pa = tile[s];
             T Az = T(0);
@@ -86,11 +104,27 @@ namespace pcfd
             if (code & kOutlet) Az += T(2) * h * pa;
             return Az;
         }
+        // The rows of the x-adjacent cells s (x even) and s + 1 of the tile; pa: their values.  The outlet
+        // is the X-max face, so only the second cell of a pair can have its bit.
+        template <class T>
+        __device__ inline Pair<T> structured_pair(const T* tile, int s, uchar2 code, T h, Pair<T>& pa)
+        {
+            pa = load_pair(tile + s);
+            const T left = tile[s - 1], right = tile[s + 2];
+            const Pair<T> ym = load_pair(tile + s - kP1), yp = load_pair(tile + s + kP1);
+            const Pair<T> zm = load_pair(tile + s - kP2), zp = load_pair(tile + s + kP2);
+            Pair<T> Az;
+            Az.x = structured_row<T>(pa.x, left, pa.y, ym.x, yp.x, zm.x, zp.x, code.x, h);
+            Az.y = structured_row<T>(pa.y, pa.x, right, ym.y, yp.y, zm.y, zp.y, code.y, h);
+            if (code.y & kOutlet) Az.y += T(2) * h * pa.y;
+            return Az;
+        }
 
         // Damping over the diagonal, w / D, of a non-deferred row: D is h per open face plus 2h
         // for the outlet, so it is looked up by (open-face count, outlet) per level.
         constexpr int kDiagonalKinds = 14;
         __device__ inline int diagonal_kind(uint8_t code) { return __popc(code & kOpenMask) + 7 * ((code >> 6) & 1); }
+        __device__ inline int inner_kind(uint8_t code) { return __popc(code & kOpenMask); }   // x even: no outlet
 
         // ---- persistent, double-buffered variant -------------------------------------------
         // Each CTA walks bricks b, b + G, ... and stages brick n+1 (tile + halos, r, codes) with
@@ -121,7 +155,7 @@ namespace pcfd
             else copy4(dst, src, valid);
         }
         __device__ inline void copy_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-        template <int N> __device__ inline void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+        template <int N> __device__ inline void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
         // What one thread needs of a brick: the head and the neighbour of the halo face it copies.
         struct Ticket
@@ -137,7 +171,7 @@ namespace pcfd
             return Ticket{h.x, h.y, h.z, h.w, m->nbr[face], m->nbase[face], int(b), v.stage_neighbour ? v.stage_neighbour[6 * b + face] : -1};
         }
 
-        template <class T, bool kWithR>
+        template <class T, bool kWithR, bool kWithCode = true>
         __device__ inline void issue_brick(const Ticket& k, const T* __restrict__ z, const T* __restrict__ r,
                                            const uint8_t* __restrict__ code, T* tile, T* rbuf, uint8_t* cbuf)
         {
@@ -148,7 +182,7 @@ namespace pcfd
                 copy_pair<T>(tile + tix(i, j, kk), z + base + c, true);
                 if (kWithR) copy_pair<T>(rbuf + rix(c), r + base + c, true);
             }
-            if (t < 32) copy16(cbuf + cix(16 * t), code + base + 16 * t, true);
+            if (kWithCode && t < 32) copy16(cbuf + cix(16 * t), code + base + 16 * t, true);
             const bool valid = k.nbr >= 0;
             const int64_t nb = int64_t(valid ? k.nbr : k.slot) * kC3;   // any valid address when zero-filling
             if (t < 128)
@@ -249,64 +283,10 @@ namespace pcfd
             double omega;
         };
 
-        // Completes deferred row d from its structured part t[a] (structured DOFs) and right-hand
-        // side r[a]: the compact-edge gather and the gauges, in the order of the unfused operator.
-        // kFinish 0: z_new into out[a], 1: residual into residual[d], 2: residual into out[a].
-        // The packed row holds every index the row needs, so its gathers are two loads deep.
-        template <int kFinish, class T, class TO, class TC, int kProlong>
-        __device__ inline void finish_row(const DeferredView& dv, int d, int64_t structured, const T* __restrict__ z,
-                                          const T* __restrict__ r, const T* __restrict__ t, const TC* __restrict__ e,
-                                          double scale, TO* __restrict__ out, double* __restrict__ residual)
-        {
-            const int4 row = dv.row[d];
-            const int a = row.x, edges = row.w >> 8, gauges = (row.w >> 2) & 63;
-            const bool on = row.w & 1, incident = row.w & 2;
-            // the prolonged iterate at DOF q with map index c (active DOFs only)
-            auto value = [&](int q, int c) {
-                double v = double(z[q]);
-                if (kProlong == 2)
-                {
-                    if (c >= 0) v += scale * double(e[c]);
-                }
-                else if (kProlong == 1)
-                {
-                    const int base = dv.aggregate[q] - dv.base_offset;
-                    if (base >= 0 && base < dv.base_cells) v += scale * double(e[base]);
-                }
-                return v;
-            };
-            // the row's independent loads first, so that they are in flight together
-            double Az = a < structured ? double(t[a]) : 0.0;
-            const double rc = double(r[a]);
-            const double D = dv.diag[a];
-            const double za = on ? value(a, row.z) : double(z[a]);
-            if (incident)
-            {
-                // the compact edges' two-point terms, coefficient * (z_a - z_other): the reference's
-                // sign * coefficient * (z_lower - z_upper) bit for bit (exact negations)
-                double sum = 0.0;
-#pragma unroll 2
-                for (int q = row.y; q < row.y + edges; ++q)
-                {
-                    const int2 other = dv.edge[q];
-                    sum += dv.edge_coefficient[q] * (za - value(other.x, other.y));
-                }
-                Az += sum;
-            }
-            if (gauges)
-                for (int g = dv.gauge_offset[d], g1 = g + gauges; g < g1; ++g) Az += dv.gauge_coefficient[g] * za;
-            if (kFinish == 0)
-            {
-                if (!on) out[a] = TO(0);
-                else out[a] = TO(D > 0.0 ? za + dv.omega * (rc - Az) / D : za);
-            }
-            else if (kFinish == 1) residual[d] = on ? rc - Az : 0.0;
-            else out[a] = TO(on ? rc - Az : 0.0);
-        }
-
         // CTAs of 256 threads the launch bounds keep resident per SM: six for the float sweeps and
-        // the FP64 operator (<= 40 registers, <= 27 KB shared memory), four for the FP64 sweeps.
-        template <int kMode, class T> constexpr int pipe_resident() { return (sizeof(T) == 4 || kMode == 2) ? 6 : 4; }
+        // the FP64 operator (<= 40 registers, <= 27 KB shared memory), four for the FP64 sweeps.  The
+        // fused pre-sweeps (kMode 4) take 48 registers in float: five.
+        template <int kMode, class T> constexpr int pipe_resident() { return kMode == 4 ? (sizeof(T) == 4 ? 5 : 4) : (sizeof(T) == 4 || kMode == 2) ? 6 : 4; }
 
         // kMode 0: Jacobi sweep, 1: residual restriction, 2: structured apply (out = A_struct z)
         // T: field type of z, r, t (double, or float for the FP32 multigrid); TO: output type.
@@ -323,6 +303,8 @@ namespace pcfd
             __shared__ __align__(16) uint8_t cbuf[2][kCSize];
             __shared__ double residual[kMode == 1 ? kC3 : 1];
             __shared__ __align__(16) TC ebuf[kProlong == 2 ? 2 : 1][kProlong == 2 ? 512 : 1];   // per thread: own, halo
+            // the WLS gradient may start beside the operator (apply_operator)
+            if (kMode == 2) chain_release();
             int64_t b = blockIdx.x;
             if (b >= bricks) return;
             const int64_t G = gridDim.x;
@@ -347,13 +329,17 @@ namespace pcfd
                 else copy_wait<0>();
                 if (kProlong) prolong_own<T, TC, kProlong == 2>(cur, e, v.prolong, tile[st], ebuf[kProlong == 2 ? st : 0]);
                 __syncthreads();
-                // ---- compute brick `cur` from buffer st.  Thread t owns cell (i, j, k) = (t & 7,
-                // t >> 5, (t >> 3 & 3) + 4 q), q = 0, 1: a warp covers one x-row of 8 cells in each
-                // of four consecutive z-planes.  With rows 12 and planes 120 tile entries apart the
-                // four rows fall on disjoint shared-memory banks (float: 32 banks, offsets 0, 24, 16,
-                // 8 words; double: each half-warp's two rows 240 words apart), so no stencil read
-                // replays (the staged rhs and codes are padded per plane for the same reason);
-                // consecutive cells of a row make 32- or 64-byte global segments.
+                // ---- compute brick `cur` from buffer st.  In the sweeps and residuals thread t owns the
+                // x-adjacent cells (2 (t & 3), j, k)
+                // and (2 (t & 3) + 1, j, k), j = t >> 5, k = t >> 2 & 7: the stencil of a pair is five
+                // two-value reads and two single ones where two separate cells take fourteen, and codes,
+                // right-hand sides and results move as pairs.  The kernel is bound by instruction issue
+                // (77 % of the issue slots at 262 instructions per thread and brick with separate cells), so
+                // those reads, and the index arithmetic per copy and store, are its time.  With rows 12
+                // and planes 120 tile entries apart the lanes served together (a half-warp in float, four
+                // planes of eight values; a quarter-warp in double, two planes) fall on disjoint
+                // shared-memory banks (the staged rhs and codes are padded per plane for the same
+                // reason); a warp's stores are 32- or 64-byte rows of the eight planes.
                 const T* F = tile[st];
                 const int l = cur.level;
                 const T h = T(v.level_h[l]);
@@ -361,34 +347,55 @@ namespace pcfd
                 const int n = l >= 3 ? 1 : (kBS >> l);
                 const int size = l >= 3 ? kC3 : (1 << (3 * l));
                 const int mask = (1 << l) - 1;
-#pragma unroll
-                for (int q = 0; q < 2; ++q)
+                if (kMode == 2)
                 {
-                    const int i = threadIdx.x & 7, j = threadIdx.x >> 5, k = ((threadIdx.x >> 3) & 3) + 4 * q;
+                    // The operator keeps one cell at a time, (t & 7, t >> 5, (t >> 3 & 3) + 4 q): it is bound by
+                    // bytes rather than issue, and the pairs' single FP64 reads share banks (16 M cells: 102
+                    // against 104 us alone, and 189 against 194 with the gradient beside it).
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                    {
+                        const int i = threadIdx.x & 7, j = threadIdx.x >> 5, k = ((threadIdx.x >> 3) & 3) + 4 * q;
+                        const int c = (k * kBS + j) * kBS + i;
+                        out[base + c] = TO(structured_cell<T>(F, tix(i, j, k), cbuf[st][cix(c)], h));
+                    }
+                }
+                else
+                {
+                    const int i = 2 * (threadIdx.x & 3), j = threadIdx.x >> 5, k = (threadIdx.x >> 2) & 7;
                     const int c = (k * kBS + j) * kBS + i;
-                    const int s = tix(i, j, k);
-                    const uint8_t code = cbuf[st][cix(c)];
-                    const T Az = structured_row<T>(F, s, code, h);
-                    if (kMode == 2) out[base + c] = TO(Az);
+                    const uchar2 code = *reinterpret_cast<const uchar2*>(cbuf[st] + cix(c));
+                    Pair<T> pa;
+                    const Pair<T> Az = structured_pair<T>(F, tix(i, j, k), code, h, pa);
+                    const Pair<T> rc = load_pair(rbuf[st] + rix(c));
+                    const bool defer_x = code.x & kDeferred, defer_y = code.y & kDeferred;
+                    if (defer_x) t[base + c] = Az.x;
+                    if (defer_y) t[base + c + 1] = Az.y;
+                    if (kMode == 1)
+                    {
+                        auto put = [&](int x, uint8_t cell_code, T rest) {
+                            const int group = l >= 3 ? 0 : ((k >> l) * n + (j >> l)) * n + (x >> l);
+                            const int within = l >= 3 ? (k * kBS + j) * kBS + x : ((((k & mask) << l) + (j & mask)) << l) + (x & mask);
+                            residual[group * size + within] = (cell_code && !(cell_code & kDeferred)) ? double(rest) : 0.0;
+                        };
+                        put(i, code.x, rc.x - Az.x);
+                        put(i + 1, code.y, rc.y - Az.y);
+                    }
                     else
                     {
-                        const T rc = rbuf[st][rix(c)];
-                        if (code & kDeferred) t[base + c] = Az;
+                        Pair<TO> result;
                         if (kMode == 0)
                         {
-                            if (!(code & kDeferred))
-                                out[base + c] = code ? TO(F[s] + (rc - Az) * damping[l * kDiagonalKinds + diagonal_kind(code)]) : TO(0);
-                        }
-                        else if (kMode == 3)
-                        {
-                            if (!(code & kDeferred)) out[base + c] = code ? TO(rc - Az) : TO(0);
+                            result.x = code.x ? TO(pa.x + (rc.x - Az.x) * damping[l * kDiagonalKinds + inner_kind(code.x)]) : TO(0);
+                            result.y = code.y ? TO(pa.y + (rc.y - Az.y) * damping[l * kDiagonalKinds + diagonal_kind(code.y)]) : TO(0);
                         }
                         else
                         {
-                            const int group = l >= 3 ? 0 : ((k >> l) * n + (j >> l)) * n + (i >> l);
-                            const int within = l >= 3 ? c : ((((k & mask) << l) + (j & mask)) << l) + (i & mask);
-                            residual[group * size + within] = (code && !(code & kDeferred)) ? double(rc - Az) : 0.0;
+                            result.x = code.x ? TO(rc.x - Az.x) : TO(0);
+                            result.y = code.y ? TO(rc.y - Az.y) : TO(0);
                         }
+                        // a deferred row's entry is written by the finish launch
+                        *reinterpret_cast<Pair<TO>*>(out + base + c) = result;
                     }
                 }
                 if (kMode == 1)
@@ -494,6 +501,140 @@ namespace pcfd
             }
         }
 
+        // The value of the first sweep from zero, w r / D; deferred rows read the assembled D.
+        template <class T>
+        __device__ inline T first_value(uint8_t code, double rq, int64_t q, int level, const T* __restrict__ damping,
+                                        const double* __restrict__ diag, double omega)
+        {
+            if (code & kDeferred)
+            {
+                const double D = diag[q];
+                return D > 0.0 ? T(omega * rq / D) : T(0);
+            }
+            return code ? T(rq) * damping[level * kDiagonalKinds + diagonal_kind(code)] : T(0);
+        }
+
+        // The two pre-sweeps in one pass: the first, from zero, is a value per cell, so its iterate is
+        // formed in the tile from r (own cells and halos) and never written; the second is the sweep
+        // of brick_pipe_kernel.  FP32 multigrid: also writes the float copy of r that the later sweeps
+        // read.  Its time is instruction issue (every halo value is formed again in each brick that reads
+        // it), so it saves a launch, not a pass: see kFusedPreBricks.
+        // r is staged in double by cp.async, double-buffered as in the pipeline; each thread turns the
+        // entries it copied itself into the iterate (no barrier between), with their code bytes
+        // prefetched into registers a brick ahead.
+        struct CodePair
+        {
+            uchar2 own, halo;
+        };
+        __device__ inline CodePair load_codes(const Ticket& k, const uint8_t* __restrict__ code)
+        {
+            const int t = threadIdx.x;
+            CodePair c;
+            c.own = *reinterpret_cast<const uchar2*>(code + int64_t(k.slot) * kC3 + 2 * t);
+            c.halo = make_uchar2(0, 0);
+            if (k.nbr < 0) return c;
+            const uint8_t* nb = code + int64_t(k.nbr) * kC3;
+            if (t < 128)
+            {
+                const int face = 2 + (t >> 5), w = t & 31;
+                const int kk = face < 4 ? w >> 2 : (face == 4 ? kBS - 1 : 0), i = face < 4 ? (w & 3) * 2 : (w * 2) & 7;
+                const int j = face < 4 ? (face == 2 ? kBS - 1 : 0) : (w * 2) >> 3;
+                c.halo = *reinterpret_cast<const uchar2*>(nb + (kk * kBS + j) * kBS + i);
+            }
+            else
+            {
+                const int u = t - 128;
+                c.halo.x = nb[(((u >> 3) & 7) * kBS + (u & 7)) * kBS + ((u >> 6) == 0 ? kBS - 1 : 0)];
+            }
+            return c;
+        }
+        template <class T, class TO>
+        __global__ void __launch_bounds__(256, pipe_resident<4, T>()) brick_first_kernel(BrickView v, int64_t bricks, const double* __restrict__ r,
+            TO* __restrict__ out, T* __restrict__ t, T* __restrict__ r_copy, const T* __restrict__ damping0, const T* __restrict__ damping,
+            const double* __restrict__ diag, double omega0)
+        {
+            __shared__ __align__(16) double rtile[2][kTileSize];
+            __shared__ __align__(16) T tile[kTileSize];
+            __shared__ __align__(16) uint8_t cbuf[kCSize];
+            int64_t b = blockIdx.x;
+            if (b >= bricks) return;
+            const int64_t G = gridDim.x;
+            const int tid = threadIdx.x;
+            auto issue = [&](const Ticket& k, double* dst) { issue_brick<double, false, false>(k, r, nullptr, nullptr, dst, nullptr, nullptr); };
+            Ticket cur = load_ticket(v, b);
+            issue(cur, rtile[0]);
+            copy_commit();
+            CodePair codes = load_codes(cur, v.code);
+            Ticket next = b + G < bricks ? load_ticket(v, b + G) : cur;
+            for (int it = 0;; ++it)
+            {
+                const int st = it & 1;
+                const bool has_next = b + G < bricks;
+                Ticket after = next;
+                CodePair next_codes = codes;
+                if (has_next)
+                {
+                    issue(next, rtile[st ^ 1]);
+                    copy_commit();
+                    next_codes = load_codes(next, v.code);
+                    if (b + 2 * G < bricks) after = load_ticket(v, b + 2 * G);
+                    copy_wait<1>();
+                }
+                else copy_wait<0>();
+                const int l = cur.level;
+                const int64_t base = int64_t(cur.slot) * kC3;
+                const double* R = rtile[st];
+                {
+                    const int c = 2 * tid, at = tix(c & 7, (c >> 3) & 7, c >> 6);
+                    tile[at] = first_value<T>(codes.own.x, R[at], base + c, l, damping0, diag, omega0);
+                    tile[at + 1] = first_value<T>(codes.own.y, R[at + 1], base + c + 1, l, damping0, diag, omega0);
+                    *reinterpret_cast<uchar2*>(cbuf + cix(c)) = codes.own;
+                    if (sizeof(T) == 4 && r_copy) *reinterpret_cast<float2*>(r_copy + base + c) = make_float2(float(R[at]), float(R[at + 1]));
+                    const int64_t nb = int64_t(cur.nbr) * kC3;
+                    if (tid < 128)
+                    {
+                        const int face = 2 + (tid >> 5), w = tid & 31;
+                        int i, j, kk, hj, hk;
+                        if (face < 4) { kk = w >> 2; i = (w & 3) * 2; j = face == 2 ? kBS - 1 : 0; hj = face == 2 ? -1 : kBS; hk = kk; }
+                        else { i = (w * 2) & 7; j = (w * 2) >> 3; kk = face == 4 ? kBS - 1 : 0; hj = j; hk = face == 4 ? -1 : kBS; }
+                        const int h = tix(i, hj, hk);
+                        const int64_t q = nb + (kk * kBS + j) * kBS + i;
+                        tile[h] = first_value<T>(codes.halo.x, R[h], q, l, damping0, diag, omega0);
+                        tile[h + 1] = first_value<T>(codes.halo.y, R[h + 1], q + 1, l, damping0, diag, omega0);
+                    }
+                    else
+                    {
+                        const int u = tid - 128, face = u >> 6, j = u & 7, kk = (u >> 3) & 7;
+                        const int h = tix(face == 0 ? -1 : kBS, j, kk);
+                        tile[h] = first_value<T>(codes.halo.x, R[h], nb + (kk * kBS + j) * kBS + (face == 0 ? kBS - 1 : 0), l, damping0, diag, omega0);
+                    }
+                }
+                __syncthreads();
+                const T h = T(v.level_h[l]);
+                {
+                    const int i = 2 * (tid & 3), j = tid >> 5, k = (tid >> 2) & 7;
+                    const int c = (k * kBS + j) * kBS + i, s = tix(i, j, k);
+                    const uchar2 code = *reinterpret_cast<const uchar2*>(cbuf + cix(c));
+                    Pair<T> pa;
+                    const Pair<T> Az = structured_pair<T>(tile, s, code, h, pa);
+                    const double2 rc = load_pair(R + s);
+                    if (code.x & kDeferred) t[base + c] = Az.x;
+                    if (code.y & kDeferred) t[base + c + 1] = Az.y;
+                    // a deferred row's entry is written by the finish launch
+                    Pair<TO> result;
+                    result.x = code.x ? TO(pa.x + (T(rc.x) - Az.x) * damping[l * kDiagonalKinds + inner_kind(code.x)]) : TO(0);
+                    result.y = code.y ? TO(pa.y + (T(rc.y) - Az.y) * damping[l * kDiagonalKinds + diagonal_kind(code.y)]) : TO(0);
+                    *reinterpret_cast<Pair<TO>*>(out + base + c) = result;
+                }
+                __syncthreads();
+                if (!has_next) break;
+                b += G;
+                cur = next;
+                next = after;
+                codes = next_codes;
+            }
+        }
+
         // Brick-local block smoother: z = x_k after k Chebyshev iterations for the brick's diagonal
         // block A_B x = r (x_0 = 0, D^-1 preconditioned), A_B = the full diagonal D minus h for every
         // open face between two cells of the brick.  D^-1 A_B is diagonally dominant, so its
@@ -563,20 +704,84 @@ namespace pcfd
             if (q < end) z[q] = active[q] && diag[q] > 0.0 ? omega * r[q] / diag[q] : 0.0;
         }
 
-        // Completes deferred rows after the pipeline launch: A_orth z = t (structured part) +
-        // compact-edge gather + gauges.  One thread per row: the rows are a sparse, irregular
-        // subset (cut cells, coarse/fine interfaces), so a launch of their own keeps every SM busy
-        // where finishing them inside the brick CTAs left most threads idle (measured slower).
-        // kMode 0: z_new, 1: residual into the compact deferred list, 2: residual into out[a]
-        template <int kMode, class T, class TO, class TC, int kProlong>
-        __global__ void __launch_bounds__(256) finish_deferred_kernel(DeferredView dv, int count, int64_t structured,
+        // Completes deferred rows after the pipeline launch: A_orth z = t (structured part, structured
+        // DOFs) + compact-edge gather + gauges, in the order of the unfused operator.  The rows are a
+        // sparse, irregular subset (cut cells, coarse/fine interfaces), so a launch of their own keeps
+        // every SM busy where finishing them inside the brick CTAs left most threads idle (measured
+        // slower).  One thread per row; the packed row holds every index the row needs.  The CTA's
+        // edges are one contiguous run: its threads first take them one each and leave the other
+        // endpoint's value and the coefficient in shared memory, so the gathers of long and short rows
+        // are all in flight together, then each row sums its own in order.
+        // kMode 0: z_new into out[a], 1: residual into the compact deferred list, 2: residual into out[a]
+        constexpr int kFinishThreads = 128, kFinishEdges = 384;
+        // kProlong 3: the iterate is the first sweep's (not stored): w0 r / D at every row here and every
+        // edge endpoint, which are deferred rows too; TR is double then, and fragments' r_copy is written.
+        template <int kMode, class T, class TO, class TC, int kProlong, class TR>
+        __global__ void __launch_bounds__(kFinishThreads) finish_deferred_kernel(DeferredView dv, int count, int64_t structured,
                                                                       const TC* __restrict__ e, double scale, const T* __restrict__ z,
-                                                                      const T* __restrict__ r, const T* __restrict__ t,
-                                                                      TO* __restrict__ out, double* __restrict__ residual)
+                                                                      const TR* __restrict__ r, const T* __restrict__ t,
+                                                                      TO* __restrict__ out, double* __restrict__ residual, T* __restrict__ r_copy)
         {
-            const int d = blockIdx.x * blockDim.x + threadIdx.x;
-            if (d >= count) return;
-            finish_row<kMode, T, TO, TC, kProlong>(dv, d, structured, z, r, t, e, scale, out, residual);
+            __shared__ double other_value[kFinishEdges], edge_coefficient[kFinishEdges];
+            const int first = blockIdx.x * kFinishThreads, d = first + threadIdx.x, top = min(count, first + kFinishThreads) - 1;
+            const bool here = d < count;
+            const int4 row = dv.row[here ? d : top], low = dv.row[first], high = dv.row[top];
+            const int begin = low.y, end = high.y + (high.w >> 8);
+            const int a = row.x, edges = here ? row.w >> 8 : 0, gauges = (row.w >> 2) & 63;
+            const bool on = row.w & 1, incident = row.w & 2;
+            // the prolonged iterate at DOF q with map index c (active DOFs only)
+            auto value = [&](int q, int c) {
+                if (kProlong == 3)
+                {
+                    const double Dq = dv.diag[q];
+                    return Dq > 0.0 ? double(T(scale * double(r[q]) / Dq)) : 0.0;
+                }
+                double v = double(z[q]);
+                if (kProlong == 2)
+                {
+                    if (c >= 0) v += scale * double(e[c]);
+                }
+                else if (kProlong == 1)
+                {
+                    const int base = dv.aggregate[q] - dv.base_offset;
+                    if (base >= 0 && base < dv.base_cells) v += scale * double(e[base]);
+                }
+                return v;
+            };
+            // the row's independent loads first, so that they are in flight together
+            double Az = a < structured ? double(t[a]) : 0.0;
+            const double rc = double(T(r[a]));
+            const double D = dv.diag[a];
+            const double za = on ? value(a, row.z) : (kProlong == 3 ? 0.0 : double(z[a]));
+            if (kProlong == 3 && r_copy && here && a >= structured) r_copy[a] = T(r[a]);
+            // the compact edges' two-point terms, coefficient * (z_a - z_other): the reference's
+            // sign * coefficient * (z_lower - z_upper) bit for bit (exact negations)
+            double sum = 0.0;
+            for (int run = begin; run < end; run += kFinishEdges)
+            {
+                const int stop = min(end, run + kFinishEdges);
+                for (int q = run + threadIdx.x; q < stop; q += kFinishThreads)
+                {
+                    const int2 other = dv.edge[q];
+                    edge_coefficient[q - run] = dv.edge_coefficient[q];
+                    other_value[q - run] = value(other.x, other.y);
+                }
+                __syncthreads();
+                for (int q = max(row.y, run), q1 = min(row.y + edges, stop); q < q1; ++q)
+                    sum += edge_coefficient[q - run] * (za - other_value[q - run]);
+                if (stop < end) __syncthreads();
+            }
+            if (!here) return;
+            if (incident) Az += sum;
+            if (gauges)
+                for (int g = dv.gauge_offset[d], g1 = g + gauges; g < g1; ++g) Az += dv.gauge_coefficient[g] * za;
+            if (kMode == 0)
+            {
+                if (!on) out[a] = TO(0);
+                else out[a] = TO(D > 0.0 ? za + dv.omega * (rc - Az) / D : za);
+            }
+            else if (kMode == 1) residual[d] = on ? rc - Az : 0.0;
+            else out[a] = TO(on ? rc - Az : 0.0);
         }
 
         // map indices of the packed deferred rows and edges (composite cycle)
@@ -909,14 +1114,17 @@ namespace pcfd
                                 s.diagonal, s.aggregate, s.base_offset, s.base_cells, omega};
         }
 
-        template <int kMode, class T, class TO, class TC, int kProlong>
-        void finish(System& s, const T* z, const T* r, TO* out, const TC* e, const T* t, double omega = 2.0 / 3.0)
+        template <int kMode, class T, class TO, class TC, int kProlong, class TR = T>
+        void finish(System& s, const T* z, const TR* r, TO* out, const TC* e, const T* t, double omega = 2.0 / 3.0, double scale = 0.0,
+                    T* r_copy = nullptr)
         {
             FineSmoother& f = s.fine;
             if (!f.deferred_count) return;
             require(kProlong != 2 || f.map_attached, "deferred rows: composite map indices not attached");
-            finish_deferred_kernel<kMode, T, TO, TC, kProlong><<<blocks_for(f.deferred_count), kThreads, 0, launch_stream(s)>>>(
-                deferred_view(s, omega), f.deferred_count, s.structured, e, s.mg_prolong_scale, z, r, t, out, f.deferred_residual);
+            finish_deferred_kernel<kMode, T, TO, TC, kProlong, TR>
+                <<<blocks_for(f.deferred_count, kFinishThreads), kFinishThreads, 0, launch_stream(s)>>>(
+                    deferred_view(s, omega), f.deferred_count, s.structured, e, kProlong == 3 ? scale : s.mg_prolong_scale, z, r, t, out,
+                    f.deferred_residual, r_copy);
         }
 
         // Persistent grid of a pipeline kernel: the system's CTAs per SM (autotuned), capped by the
@@ -964,15 +1172,32 @@ namespace pcfd
                 view(s), s.active_bricks, z, r, out, w.t, e, nullptr, damping);
             finish<0, T, TO, TC, kProlong>(s, z, r, out, e, w.t, omega);
         }
-        // the first pre-sweep from z = 0 (slot 0 of the schedule when it is on)
-        template <class T> void first_sweep(System& s, const double* r, T* z, T* r_copy)
+        // Up to this many bricks the two pre-sweeps run as one launch (one preconditioner application on
+        // 65 k cells 45.2 against 49.2 us, on 1.1 M 161.6 and 162.0); above, the first is a pass of its own
+        // (4.2 M 293.6 and 291.9, 16 M 882 and 867).
+        constexpr int kFusedPreBricks = 4096;
+        // the two pre-sweeps from z = 0 (slots 0 and 1 of the schedule, else w = 2/3) into out; first: a
+        // buffer for the first sweep's iterate; r_copy: the float copy of r (FP32 multigrid)
+        template <class T, class TC> void pre_sweeps(System& s, const double* r, T* first, T* out, T* r_copy, bool schedule)
         {
             FineSmoother& f = s.fine;
             FineBuffers<T> w(f);
-            const bool cheb = w.chebyshev != nullptr;
-            first_sweep_kernel<T><<<blocks_for((int64_t(s.S) + 3) / 4), kThreads, 0, launch_stream(s)>>>(
-                f.code, s.brick_level, cheb ? w.chebyshev : w.damping, s.diagonal, s.active, r, z, r_copy, s.structured, s.S,
-                cheb ? f.cheb_omega[0] : 2.0 / 3.0);
+            const bool cheb = schedule && w.chebyshev;
+            const T* damping0 = cheb ? w.chebyshev : w.damping;
+            const double omega0 = cheb ? f.cheb_omega[0] : 2.0 / 3.0;
+            if (s.active_bricks > kFusedPreBricks)
+            {
+                first_sweep_kernel<T><<<blocks_for((int64_t(s.S) + 3) / 4), kThreads, 0, launch_stream(s)>>>(
+                    f.code, s.brick_level, damping0, s.diagonal, s.active, r, first, r_copy, s.structured, s.S, omega0);
+                if constexpr (std::is_same<T, float>::value) sweep<T, T, TC, 0>(s, first, r_copy, out, nullptr, cheb ? 1 : -1);
+                else sweep<T, T, TC, 0>(s, first, r, out, nullptr, cheb ? 1 : -1);
+                return;
+            }
+            const T* damping1 = cheb ? w.chebyshev + f.cheb_stride : w.damping;
+            const double omega1 = cheb ? f.cheb_omega[1] : 2.0 / 3.0;
+            brick_first_kernel<T, T><<<pipe_grid<4, T>(s), 256, 0, launch_stream(s)>>>(view(s), s.active_bricks, r, out, w.t, r_copy, damping0,
+                                                                                       damping1, s.diagonal, omega0);
+            finish<0, T, T, TC, 3, double>(s, nullptr, r, out, static_cast<const TC*>(nullptr), w.t, omega1, omega0, r_copy);
         }
 
         template <class T>
@@ -1011,9 +1236,7 @@ namespace pcfd
         if (std::is_same<TC, float>::value && f.z32.n)
         {
             float *a = f.z32.p, *b = f.z32b.p, *r32 = f.r32.p;
-            first_sweep_kernel<float><<<blocks_for((int64_t(s.S) + 3) / 4), kThreads, 0, launch_stream(s)>>>(
-                f.code, s.brick_level, f.damping32.p, s.diagonal, s.active, r, a, r32, s.structured, s.S, 2.0 / 3.0);
-            sweep<float, float, TC, 0>(s, a, r32, b, nullptr);
+            pre_sweeps<float, TC>(s, r, a, b, r32, false);
             coarse(b, r32);
             sweep<float, float, TC, 1>(s, b, r32, a, base.x.p);
             sweep<float, double, TC, 0>(s, a, r32, z, nullptr);
@@ -1021,9 +1244,7 @@ namespace pcfd
         else
         {
             double* a = f.z.p;
-            first_sweep_kernel<double><<<blocks_for((int64_t(s.S) + 3) / 4), kThreads, 0, launch_stream(s)>>>(
-                f.code, s.brick_level, f.damping.p, s.diagonal, s.active, r, a, nullptr, s.structured, s.S, 2.0 / 3.0);
-            sweep<double, double, TC, 0>(s, a, r, z, nullptr);
+            pre_sweeps<double, TC>(s, r, a, z, nullptr, false);
             coarse(z, r);
             sweep<double, double, TC, 1>(s, z, r, a, base.x.p);
             sweep<double, double, TC, 0>(s, a, r, z, nullptr);
@@ -1103,9 +1324,7 @@ namespace pcfd
                 composite_tail<TC>(s, r, z, first);
                 return;
             }
-            double* a = f.z.p;
-            first_sweep<double>(s, r, a, nullptr);
-            sweep<double, double, TC, 0>(s, a, r, z, nullptr, 1);
+            pre_sweeps<double, TC>(s, r, f.z.p, z, nullptr, true);
             composite_tail<TC>(s, r, z, first);
         }
     }
@@ -1155,8 +1374,7 @@ namespace pcfd
         {
             FineSmoother& f = s.fine;
             float *a = f.z32.p, *b = f.z32b.p, *r32 = f.r32.p, *res = f.res32.p;
-            first_sweep<float>(s, r, a, r32);
-            sweep<float, float, float, 0>(s, a, r32, b, nullptr, 1);
+            pre_sweeps<float, float>(s, r, a, b, r32, true);
             brick_pipe_kernel<3, float, float, float, 0><<<pipe_grid<3, float>(s), 256, 0, launch_stream(s)>>>(
                 view(s), s.active_bricks, b, r32, res, f.t32.p, nullptr, nullptr, f.damping32.p);
             finish<2, float, float, float, 0>(s, b, r32, res, static_cast<const float*>(nullptr), f.t32.p);
@@ -1191,9 +1409,7 @@ namespace pcfd
         double* a = f.z.p;
         if (stage == 0)
         {
-            first_sweep_kernel<double><<<blocks_for((int64_t(s.S) + 3) / 4), kThreads, 0, launch_stream(s)>>>(
-                f.code, s.brick_level, f.damping.p, s.diagonal, s.active, r, a, nullptr, s.structured, s.S, 2.0 / 3.0);
-            sweep<double, double, double, 0>(s, a, r, z, nullptr);
+            pre_sweeps<double, double>(s, r, a, z, nullptr, false);
         }
         else if (stage == 1)
         {
