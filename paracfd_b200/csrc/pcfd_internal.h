@@ -82,17 +82,16 @@ namespace pcfd
     // Compact non-orthogonal / two-point edge set used by the irregular operator gather.
     struct IrregularOperator
     {
-        int incident_dofs = 0, connection_count = 0, regular_count = 0;
-        DBuf<int> incident_dof, incident_offset, incident_edge;
-        DBuf<int8_t> incident_sign;
-        // the same incidence entries packed for the two-point sums: the edge's other endpoint and
-        // its coefficient, so coefficient * (p[dof] - p[other]) equals sign * coefficient *
-        // (p[lower] - p[upper]) bit for bit with one load chain less
-        DBuf<int> incident_other;
+        // Incidence rows: per DOF with compact edges (connections then regular corrections, with active
+        // endpoints), its entries in order.  An entry holds all a row's sums need: the edge's other
+        // endpoint and its coefficient, so coefficient * (p[dof] - p[other]) equals sign * coefficient *
+        // (p[lower] - p[upper]) bit for bit; its gradient nodes (or -1, -1), correction, upper weight
+        // and signed open area.
+        int incident_dofs = 0, regular_count = 0;
+        DBuf<int> incident_dof, incident_offset, incident_other;
         DBuf<double> incident_coefficient;
-        // connections (coarse/fine then embedded), geometrically ordered endpoints
-        DBuf<int> conn_lower, conn_upper, conn_lower_node, conn_upper_node;
-        DBuf<double> conn_coefficient, conn_correction, conn_upper_weight, conn_area;
+        DBuf<int2> incident_nodes;
+        DBuf<double> incident_correction;       // [entries][5]
         // regular corrections
         DBuf<int> reg_lower, reg_upper, reg_lower_node, reg_upper_node;
         DBuf<double> reg_coefficient, reg_correction, reg_upper_weight, reg_area, reg_delta;
@@ -209,6 +208,7 @@ namespace pcfd
         double value[kMaxSet] = {};
     };
 
+    struct Download;   // pinned staging of large downloads (download.cu)
     struct System
     {
         // sizes
@@ -281,12 +281,12 @@ namespace pcfd
         int recycle_limit = recycle_capacity;      // recycled pairs kept between solves (pcfd_options)
         DBuf<double> dot_partial;               // reduction scratch
         DBuf<double> block_partial;             // [592][kMaxSet + 1] block-kernel partial sums
-        DBuf<double> block_result;              // [4][kMaxSet + 1] device coefficients / norms
+        DBuf<double> block_result;              // [6][kMaxSet + 1] device coefficients / norms, two columns' sets
         DBuf<double> dcgs_partial, dcgs_result; // delayed CGS2 partials [592][2 kMaxSet + 4] and coefficients
         DBuf<double> dcgs_total;                // [2 kMaxSet + 4] the partials' sums
         DBuf<unsigned> dcgs_ticket;             // CTAs of the sum kernel done (0 between launches)
         double* pinned_dcgs = nullptr;          // pinned host copies of dcgs_result, two columns
-        cudaEvent_t dcgs_ready[2] = {};         // readback of column j lands in slot j & 1
+        cudaEvent_t dcgs_ready[2] = {};         // readback of column j has landed in slot j & 1
         bool delayed_orthogonalisation = false; // pcfd_options.gmres_delayed
         double* pinned_block = nullptr;         // pinned host copy of block_result
         DBuf<double> dot_result;                // device scalars
@@ -339,6 +339,7 @@ namespace pcfd
         void* apertures = nullptr;              // MAC-mode compact aperture transport state (mac_apertures.cu)
         int momentum_mode = PCFD_MOMENTUM_CELL; // pcfd_momentum_mode of pcfd_core_initialize / step
         DBuf<float> slice_buffer;               // device output of pcfd_sample_slice_host
+        std::shared_ptr<Download> download;
         cudaEvent_t markers[8] = {};
         int64_t launches = 0;                   // kernels launched on the system stream so far
         // per-launch event pairs around one instrumented region (PCFD_PROFILE_*), for the roofline
@@ -409,6 +410,10 @@ namespace pcfd
         }
     };
 
+    // Copies a large buffer to pageable host memory on several threads; false (nothing done) for small
+    // copies and pinned destinations.  Complete when it returns (download.cu).
+    bool threaded_download(System& s, void* dst, const void* src, size_t bytes);
+
     // ---- kernels / launchers (pressure.cu) ----
     void launch_apply(System& s, const double* p, double* out, bool orthogonal_only);
     // same operator with the WLS gradient scratch in a static device array (pressure.cu)
@@ -458,7 +463,7 @@ namespace pcfd
     double learned_evaluate(System& s, int n, const float* x, const float* target, float* zhat, float* gradients);
     // vector helpers
     void vec_copy_active(System& s, const double* src, double* dst);
-    void vec_subtract(System& s, double* residual, const double* value);   // r = active ? r - v : 0
+    double vec_residual_dot(System& s, const double* b, const double* Ax, double* r);   // r = active ? b - Ax : 0; r.r
     void vec_axpy_active(System& s, double* y, const double* x, double a);
     void vec_scaled_copy_active(System& s, double* dst, const double* src, double a);
     void vec_zero(System& s, double* x);

@@ -144,51 +144,37 @@ namespace pcfd
             if (q < end) x[q] = 0.0;
         }
 
-        // Deterministic per-DOF gather of the compact two-point edges (connections first, then
-        // regular corrections), reference amr_pressure.cu:105-134 with FP64 coefficients.
-        // Two-point fluxes of the compact edges at each incident DOF, in the reference's per-DOF
-        // order (amr_pressure.cu:105-134): sign * coefficient * (p[lower] - p[upper]), evaluated as
-        // coefficient * (p[dof] - p[other]) from the packed incidence entries (equal bit for bit:
-        // negating a difference or a product is exact).
-        __global__ void irregular_orthogonal_gather_kernel(
-            const int* __restrict__ incident_dof, const int* __restrict__ incident_offset,
-            const int* __restrict__ incident_other, const double* __restrict__ incident_coefficient, int incident_dofs,
-            const uint8_t* __restrict__ active, const double* __restrict__ p, double* __restrict__ out)
-        {
-            const int node = blockIdx.x * blockDim.x + threadIdx.x;
-            if (node >= incident_dofs) return;
-            const int dof = incident_dof[node], q0 = incident_offset[node], q1 = incident_offset[node + 1];
-            const double centre = p[dof];
-            double sum = 0.0;
-#pragma unroll 2
-            for (int q = q0; q < q1; ++q)
-            {
-                const int other = incident_other[q];
-                if (active[other]) sum += incident_coefficient[q] * (centre - p[other]);
-            }
-            out[dof] += sum;
-        }
-
-        __global__ void reconstruct_gradient_kernel(const int* __restrict__ dof, const int* __restrict__ offset,
+        // WLS pressure gradient of every node, a thread per node (FP64 sums in stencil order).  Reads p only,
+        // so it may run beside the structured operator that precedes it on the stream
+        // (apply_operator); its last CTA waits for that launch, so that what follows this one finds both
+        // complete.  Bound by the scattered reads of p (32-byte sectors for 8-byte values) beside 28 B
+        // per entry: four entries in flight per thread.  Staging a CTA's entries in shared memory, one per
+        // thread, measured slower (88 against 72 us for 1.2 M nodes).
+        constexpr int kRowThreads = 128;
+        __global__ void __launch_bounds__(kRowThreads) reconstruct_gradient_kernel(const int* __restrict__ dof, const int* __restrict__ offset,
             const int* __restrict__ neighbour, const double* __restrict__ weight, const double* __restrict__ p,
             double* __restrict__ gradient, int nodes)
         {
-            const int node = blockIdx.x * blockDim.x + threadIdx.x;
-            if (node >= nodes) return;
-            const int q0 = offset[node], q1 = offset[node + 1];
-            const double centre = p[dof[node]];
-            double gx = 0, gy = 0, gz = 0;
-#pragma unroll 2
-            for (int q = q0; q < q1; ++q)
+            chain_release();
+            const int node = blockIdx.x * kRowThreads + threadIdx.x;
+            if (node < nodes)
             {
-                const double d = p[neighbour[q]] - centre;
-                gx += weight[3 * q] * d;
-                gy += weight[3 * q + 1] * d;
-                gz += weight[3 * q + 2] * d;
+                const int q0 = offset[node], q1 = offset[node + 1];
+                const double centre = p[dof[node]];
+                double gx = 0, gy = 0, gz = 0;
+#pragma unroll 4
+                for (int q = q0; q < q1; ++q)
+                {
+                    const double d = p[neighbour[q]] - centre;
+                    gx += weight[3 * q] * d;
+                    gy += weight[3 * q + 1] * d;
+                    gz += weight[3 * q + 2] * d;
+                }
+                gradient[3 * node] = gx;
+                gradient[3 * node + 1] = gy;
+                gradient[3 * node + 2] = gz;
             }
-            gradient[3 * node] = gx;
-            gradient[3 * node + 1] = gy;
-            gradient[3 * node + 2] = gz;
+            if (blockIdx.x == gridDim.x - 1) chain_wait();
         }
 
         __device__ inline double face_derivative(const double* gradient, int lower_node, int upper_node,
@@ -201,45 +187,39 @@ namespace pcfd
             return derivative;
         }
 
-        // WLS affine-exact non-orthogonal correction gather (amr_pressure.cu:135-178).
-        __global__ void irregular_nonorthogonal_gather_kernel(
-            const int* __restrict__ incident_dof, const int* __restrict__ incident_offset,
-            const int* __restrict__ incident_edge, const int8_t* __restrict__ incident_sign, int incident_dofs,
-            int connection_count, const int* __restrict__ conn_lower, const int* __restrict__ conn_upper,
-            const int* __restrict__ conn_lower_node, const int* __restrict__ conn_upper_node,
-            const double* __restrict__ conn_correction, const double* __restrict__ conn_upper_weight,
-            const double* __restrict__ conn_area, const int* __restrict__ reg_lower, const int* __restrict__ reg_upper,
-            const int* __restrict__ reg_lower_node, const int* __restrict__ reg_upper_node,
-            const double* __restrict__ reg_correction, const double* __restrict__ reg_upper_weight,
-            const double* __restrict__ reg_area, const double* __restrict__ gradient,
-            const uint8_t* __restrict__ active, double* __restrict__ out)
+        // Fluxes of the compact edges at each incident DOF (reference amr_pressure.cu:105-178), a thread per
+        // DOF: the two-point sum in the reference's per-DOF order, sign * coefficient * (p[lower] -
+        // p[upper]) evaluated as coefficient * (p[dof] - p[other]) (equal bit for bit: negating a
+        // difference or a product is exact), then with kCorrected the WLS affine-exact non-orthogonal
+        // corrections, out += each sum.  Entries have active endpoints only (build_operator drops the
+        // others) and hold everything but the values, so a row is three loads deep; as two launches
+        // over edge-indexed arrays the sums took 30 us against 21 for the 297 k DOFs of a 5.1 M-cell grid.
+        template <bool kCorrected>
+        __global__ void __launch_bounds__(kRowThreads) irregular_gather_kernel(const int* __restrict__ incident_dof,
+            const int* __restrict__ incident_offset, const int* __restrict__ incident_other, const double* __restrict__ incident_coefficient,
+            const int2* __restrict__ incident_nodes, const double* __restrict__ incident_correction, int incident_dofs,
+            const double* __restrict__ p, const double* __restrict__ gradient, double* __restrict__ out)
         {
-            const int node = blockIdx.x * blockDim.x + threadIdx.x;
+            chain_wait();
+            chain_release();
+            const int node = blockIdx.x * kRowThreads + threadIdx.x;
             if (node >= incident_dofs) return;
             const int dof = incident_dof[node], q0 = incident_offset[node], q1 = incident_offset[node + 1];
-            double sum = 0.0;
+            const double centre = p[dof], before = out[dof];
+            double two_point = 0.0, correction = 0.0;
+#pragma unroll 2
             for (int q = q0; q < q1; ++q)
             {
-                const int e = incident_edge[q];
-                int a, b, ln, un;
-                const double* corr;
-                double uw, area;
-                if (e < connection_count)
+                two_point += incident_coefficient[q] * (centre - p[incident_other[q]]);
+                if (kCorrected)
                 {
-                    a = conn_lower[e]; b = conn_upper[e]; ln = conn_lower_node[e]; un = conn_upper_node[e];
-                    corr = conn_correction + 3 * e; uw = conn_upper_weight[e]; area = conn_area[e];
+                    const int2 n = incident_nodes[q];
+                    const double* c = incident_correction + 5 * int64_t(q);
+                    const double corr[3] = {c[0], c[1], c[2]}, upper_weight = c[3], signed_area = c[4];
+                    correction += n.x >= 0 ? -signed_area * face_derivative(gradient, n.x, n.y, corr, upper_weight) : 0.0;
                 }
-                else
-                {
-                    const int r = e - connection_count;
-                    a = reg_lower[r]; b = reg_upper[r]; ln = reg_lower_node[r]; un = reg_upper_node[r];
-                    corr = reg_correction + 3 * r; uw = reg_upper_weight[r]; area = reg_area[r];
-                }
-                if (!active[a] || !active[b] || ln < 0 || un < 0) continue;
-                const double flux = -area * face_derivative(gradient, ln, un, corr, uw);
-                sum += double(incident_sign[q]) * flux;
             }
-            out[dof] += sum;
+            out[dof] = kCorrected ? (before + two_point) + correction : before + two_point;
         }
 
         __global__ void gauge_apply_kernel(const int* dof, const double* coefficient, int count, const double* p, double* out)
@@ -249,41 +229,58 @@ namespace pcfd
         }
     }
 
+    namespace
+    {
+        // The operator with the WLS-gradient scratch at `gradient`.  Its parts: the structured 7-point part
+        // (reads p, writes out), the gradient (reads p) and the compact edges (add to out).  The brick
+        // kernel's persistent CTAs release their successor at once and the gradient does not read what
+        // they write, so the two run side by side; the edges follow when both are complete.  Grids
+        // without compact edges need no gradient.  One application, before -> now: 65 k cells on one level
+        // 8.2 -> 4.1 us, 1.1 M on three levels 38 -> 28, 5.1 M 88 -> 68, 16 M on four 220 -> 189.
+        void apply_operator(System& s, const double* p, double* out, bool orthogonal_only, double* gradient)
+        {
+            IrregularOperator& o = s.irr;
+            if (s.S > s.structured)
+                zero_range_kernel<<<blocks_for(s.S - s.structured), kThreads, 0, launch_stream(s)>>>(out, s.structured, s.S);
+            bool beside = false;       // the gradient may start while the structured part runs
+            if (s.active_bricks)
+            {
+                ProfileScope scope(s, PCFD_PROFILE_STRUCTURED_APPLY);
+                if (s.fine.enabled && aligned16(p) && aligned16(out))
+                {
+                    brick_apply(s, p, out);
+                    beside = !scope.on;
+                }
+                else if (s.bs == 8)
+                    structured_apply8_kernel<double><<<s.active_bricks, 256, 0, launch_stream(s)>>>(
+                        s.active_brick_list, s.brick_level, s.brick_nbr, s.brick_flags, s.d_level_h, s.active,
+                        s.cut_face_mask, p, out, s.outlet ? 1 : 0);
+                else
+                    structured_apply_generic_kernel<double><<<blocks_for(int64_t(s.active_bricks) * s.bs3), kThreads, 0, launch_stream(s)>>>(
+                        s.active_brick_list, s.active_bricks, s.bs, s.brick_level, s.brick_nbr, s.brick_flags, s.d_level_h,
+                        s.active, s.cut_face_mask, p, out, s.outlet ? 1 : 0);
+            }
+            const bool corrected = !orthogonal_only && o.gradient_nodes && o.incident_dofs;
+            if (corrected && beside)
+                launch_chained(s, reconstruct_gradient_kernel, unsigned(blocks_for(o.gradient_nodes, kRowThreads)), kRowThreads, o.grad_dof,
+                               o.grad_offset, o.grad_neighbour, o.grad_weight, p, gradient, o.gradient_nodes);
+            else if (corrected)
+                reconstruct_gradient_kernel<<<blocks_for(o.gradient_nodes, kRowThreads), kRowThreads, 0, launch_stream(s)>>>(
+                    o.grad_dof, o.grad_offset, o.grad_neighbour, o.grad_weight, p, gradient, o.gradient_nodes);
+            if (o.gauges)
+                gauge_apply_kernel<<<blocks_for(o.gauges), kThreads, 0, launch_stream(s)>>>(o.gauge_dof, o.gauge_coefficient, o.gauges, p, out);
+            if (o.incident_dofs)
+                launch_chained(s, corrected ? irregular_gather_kernel<true> : irregular_gather_kernel<false>,
+                               unsigned(blocks_for(o.incident_dofs, kRowThreads)), kRowThreads, o.incident_dof, o.incident_offset,
+                               o.incident_other, o.incident_coefficient, o.incident_nodes, o.incident_correction, o.incident_dofs, p,
+                               gradient, out);
+            cuda_check(cudaGetLastError(), "launch pressure operator");
+        }
+    }
+
     void launch_apply(System& s, const double* p, double* out, bool orthogonal_only)
     {
-        if (s.active_bricks)
-        {
-            ProfileScope scope(s, PCFD_PROFILE_STRUCTURED_APPLY);
-            if (s.fine.enabled && aligned16(p) && aligned16(out)) brick_apply(s, p, out);
-            else if (s.bs == 8)
-                structured_apply8_kernel<double><<<s.active_bricks, 256, 0, launch_stream(s)>>>(
-                    s.active_brick_list, s.brick_level, s.brick_nbr, s.brick_flags, s.d_level_h, s.active,
-                    s.cut_face_mask, p, out, s.outlet ? 1 : 0);
-            else
-                structured_apply_generic_kernel<double><<<blocks_for(int64_t(s.active_bricks) * s.bs3), kThreads, 0, launch_stream(s)>>>(
-                    s.active_brick_list, s.active_bricks, s.bs, s.brick_level, s.brick_nbr, s.brick_flags, s.d_level_h,
-                    s.active, s.cut_face_mask, p, out, s.outlet ? 1 : 0);
-        }
-        if (s.S > s.structured)
-            zero_range_kernel<<<blocks_for(s.S - s.structured), kThreads, 0, launch_stream(s)>>>(out, s.structured, s.S);
-        IrregularOperator& o = s.irr;
-        if (o.incident_dofs)
-            irregular_orthogonal_gather_kernel<<<blocks_for(o.incident_dofs), kThreads, 0, launch_stream(s)>>>(
-                o.incident_dof, o.incident_offset, o.incident_other, o.incident_coefficient, o.incident_dofs, s.active, p, out);
-        if (o.gauges)
-            gauge_apply_kernel<<<blocks_for(o.gauges), kThreads, 0, launch_stream(s)>>>(o.gauge_dof, o.gauge_coefficient, o.gauges, p, out);
-        if (!orthogonal_only && o.gradient_nodes)
-        {
-            reconstruct_gradient_kernel<<<blocks_for(o.gradient_nodes), kThreads, 0, launch_stream(s)>>>(
-                o.grad_dof, o.grad_offset, o.grad_neighbour, o.grad_weight, p, o.gradient, o.gradient_nodes);
-            if (o.incident_dofs)
-                irregular_nonorthogonal_gather_kernel<<<blocks_for(o.incident_dofs), kThreads, 0, launch_stream(s)>>>(
-                    o.incident_dof, o.incident_offset, o.incident_edge, o.incident_sign, o.incident_dofs, o.connection_count,
-                    o.conn_lower, o.conn_upper, o.conn_lower_node, o.conn_upper_node, o.conn_correction, o.conn_upper_weight,
-                    o.conn_area, o.reg_lower, o.reg_upper, o.reg_lower_node, o.reg_upper_node, o.reg_correction,
-                    o.reg_upper_weight, o.reg_area, o.gradient, s.active, out);
-        }
-        cuda_check(cudaGetLastError(), "launch pressure operator");
+        apply_operator(s, p, out, orthogonal_only, s.irr.gradient);
     }
 
     // ==================================================================================
@@ -318,6 +315,22 @@ namespace pcfd
             v = block_sum(v, shared);
             if (threadIdx.x == 0) partial[blockIdx.x] = v;
         }
+        // r = b - Ax on the active entries (0 elsewhere) and its dot partials in one pass, in the order of
+        // dot_partial_kernel
+        __global__ void __launch_bounds__(256) residual_dot_kernel(const double* __restrict__ b, const double* __restrict__ Ax,
+            const uint8_t* __restrict__ active, int64_t n, double* __restrict__ r, double* __restrict__ partial)
+        {
+            __shared__ double shared[8];
+            double v = 0.0;
+            for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += int64_t(gridDim.x) * blockDim.x)
+            {
+                const double value = active[q] ? b[q] - Ax[q] : 0.0;
+                r[q] = value;
+                if (active[q]) v += value * value;
+            }
+            v = block_sum(v, shared);
+            if (threadIdx.x == 0) partial[blockIdx.x] = v;
+        }
         __global__ void __launch_bounds__(256) dot_final_kernel(const double* __restrict__ partial, int count, double* __restrict__ result)
         {
             __shared__ double shared[8];
@@ -328,13 +341,28 @@ namespace pcfd
         }
     }
 
+    namespace
+    {
+        double dot_total(System& s)
+        {
+            dot_final_kernel<<<1, 256, 0, launch_stream(s)>>>(s.dot_partial, kDotBlocks, s.dot_result);
+            cuda_check(cudaMemcpyAsync(s.pinned, s.dot_result, sizeof(double), cudaMemcpyDeviceToHost, s.stream), "dot readback");
+            cuda_check(cudaStreamSynchronize(s.stream), "dot synchronize");
+            return s.pinned[0];
+        }
+    }
+
     double device_dot(System& s, const double* a, const double* b)
     {
         dot_partial_kernel<<<kDotBlocks, 256, 0, launch_stream(s)>>>(a, b, s.active, s.S, s.dot_partial);
-        dot_final_kernel<<<1, 256, 0, launch_stream(s)>>>(s.dot_partial, kDotBlocks, s.dot_result);
-        cuda_check(cudaMemcpyAsync(s.pinned, s.dot_result, sizeof(double), cudaMemcpyDeviceToHost, s.stream), "dot readback");
-        cuda_check(cudaStreamSynchronize(s.stream), "dot synchronize");
-        return s.pinned[0];
+        return dot_total(s);
+    }
+
+    // One pass in place of a copy, a subtraction and a dot: 25 B per entry against 66.
+    double vec_residual_dot(System& s, const double* b, const double* Ax, double* r)
+    {
+        residual_dot_kernel<<<kDotBlocks, 256, 0, launch_stream(s)>>>(b, Ax, s.active, s.S, r, s.dot_partial);
+        return dot_total(s);
     }
 
     // ==================================================================================
@@ -346,11 +374,6 @@ namespace pcfd
         {
             const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
             if (q < n) dst[q] = active[q] ? src[q] : 0.0;
-        }
-        __global__ void subtract_kernel(double* r, const double* v, const uint8_t* active, int64_t n)
-        {
-            const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (q < n) r[q] = active[q] ? r[q] - v[q] : 0.0;
         }
         __global__ void axpy_active_kernel(double* y, const double* x, double a, const uint8_t* active, int64_t n)
         {
@@ -377,10 +400,6 @@ namespace pcfd
     void vec_copy_active(System& s, const double* src, double* dst)
     {
         copy_active_kernel<<<blocks_for(s.S), kThreads, 0, launch_stream(s)>>>(src, dst, s.active, s.S);
-    }
-    void vec_subtract(System& s, double* r, const double* v)
-    {
-        subtract_kernel<<<blocks_for(s.S), kThreads, 0, launch_stream(s)>>>(r, v, s.active, s.S);
     }
     void vec_axpy_active(System& s, double* y, const double* x, double a)
     {
@@ -420,7 +439,6 @@ namespace pcfd
     {
         IrregularOperator& o = s.irr;
         const int cf = t.coarse_fine.count, eb = t.embedded.count, nc = cf + eb;
-        o.connection_count = nc;
         std::vector<int> lower(nc), upper(nc), lnode(nc), unode(nc);
         std::vector<double> coefficient(nc), correction(size_t(nc) * 3), weight(nc), area(nc);
         for (int e = 0; e < nc; ++e)
@@ -437,9 +455,6 @@ namespace pcfd
             weight[e] = c.upper_gradient_weight[q];
             area[e] = c.open_area[q];
         }
-        o.conn_lower.upload(lower); o.conn_upper.upload(upper); o.conn_coefficient.upload(coefficient);
-        o.conn_lower_node.upload(lnode); o.conn_upper_node.upload(unode); o.conn_correction.upload(correction);
-        o.conn_upper_weight.upload(weight); o.conn_area.upload(area);
 
         const pcfd_regular_corrections& rc = t.regular;
         o.regular_count = rc.count;
@@ -473,23 +488,27 @@ namespace pcfd
             if (a.edge != b.edge) return a.edge < b.edge;
             return a.sign < b.sign;
         });
-        std::vector<int> idof, ioff, iedge, iother;
-        std::vector<int8_t> isign;
-        std::vector<double> icoef;
+        std::vector<int> idof, ioff, iother;
+        std::vector<int2> inodes;
+        std::vector<double> icoef, icorr;
         for (size_t q = 0; q < inc.size(); ++q)
         {
             if (q == 0 || inc[q].dof != inc[q - 1].dof) { idof.push_back(inc[q].dof); ioff.push_back(int(q)); }
-            iedge.push_back(inc[q].edge);
-            isign.push_back(inc[q].sign);
-            const int e = inc[q].edge;
-            const int lo = e < nc ? lower[e] : rl[e - nc], hi = e < nc ? upper[e] : ru[e - nc];
+            const int e = inc[q].edge, r = e - nc;
+            const bool connection = e < nc;
+            const int lo = connection ? lower[e] : rl[r], hi = connection ? upper[e] : ru[r];
             iother.push_back(inc[q].sign > 0 ? hi : lo);
-            icoef.push_back(e < nc ? coefficient[e] : rcoef[e - nc]);
+            icoef.push_back(connection ? coefficient[e] : rcoef[r]);
+            const int ln = connection ? lnode[e] : rln[r], un = connection ? unode[e] : run[r];
+            inodes.push_back(ln >= 0 && un >= 0 ? make_int2(ln, un) : make_int2(-1, -1));
+            const double* c = connection ? &correction[3 * size_t(e)] : &rcorr[3 * size_t(r)];
+            icorr.insert(icorr.end(), {c[0], c[1], c[2], connection ? weight[e] : rw[r], inc[q].sign * (connection ? area[e] : ra[r])});
         }
         ioff.push_back(int(inc.size()));
         o.incident_dofs = int(idof.size());
-        o.incident_dof.upload(idof); o.incident_offset.upload(ioff); o.incident_edge.upload(iedge); o.incident_sign.upload(isign);
+        o.incident_dof.upload(idof); o.incident_offset.upload(ioff);
         o.incident_other.upload(iother); o.incident_coefficient.upload(icoef);
+        o.incident_nodes.upload(inodes); o.incident_correction.upload(icorr);
 
         o.gradient_nodes = t.gradient_node_count;
         if (o.gradient_nodes)
@@ -566,37 +585,6 @@ namespace pcfd
             throw Error(PCFD_INVALID_ARG, "pcfd_pressure_apply_device_noalloc: " + std::to_string(o.gradient_nodes) +
                                               " WLS gradient nodes exceed the static scratch maximum of " +
                                               std::to_string(kNoAllocGradientNodes));
-        double* gradient = !orthogonal_only && o.gradient_nodes ? noalloc_scratch(s) : nullptr;
-        if (s.active_bricks)
-        {
-            if (s.fine.enabled && aligned16(p) && aligned16(out)) brick_apply(s, p, out);
-            else if (s.bs == 8)
-                structured_apply8_kernel<double><<<s.active_bricks, 256, 0, launch_stream(s)>>>(
-                    s.active_brick_list, s.brick_level, s.brick_nbr, s.brick_flags, s.d_level_h, s.active,
-                    s.cut_face_mask, p, out, s.outlet ? 1 : 0);
-            else
-                structured_apply_generic_kernel<double><<<blocks_for(int64_t(s.active_bricks) * s.bs3), kThreads, 0, launch_stream(s)>>>(
-                    s.active_brick_list, s.active_bricks, s.bs, s.brick_level, s.brick_nbr, s.brick_flags, s.d_level_h,
-                    s.active, s.cut_face_mask, p, out, s.outlet ? 1 : 0);
-        }
-        if (s.S > s.structured)
-            zero_range_kernel<<<blocks_for(s.S - s.structured), kThreads, 0, launch_stream(s)>>>(out, s.structured, s.S);
-        if (o.incident_dofs)
-            irregular_orthogonal_gather_kernel<<<blocks_for(o.incident_dofs), kThreads, 0, launch_stream(s)>>>(
-                o.incident_dof, o.incident_offset, o.incident_other, o.incident_coefficient, o.incident_dofs, s.active, p, out);
-        if (o.gauges)
-            gauge_apply_kernel<<<blocks_for(o.gauges), kThreads, 0, launch_stream(s)>>>(o.gauge_dof, o.gauge_coefficient, o.gauges, p, out);
-        if (!orthogonal_only && o.gradient_nodes)
-        {
-            reconstruct_gradient_kernel<<<blocks_for(o.gradient_nodes), kThreads, 0, launch_stream(s)>>>(
-                o.grad_dof, o.grad_offset, o.grad_neighbour, o.grad_weight, p, gradient, o.gradient_nodes);
-            if (o.incident_dofs)
-                irregular_nonorthogonal_gather_kernel<<<blocks_for(o.incident_dofs), kThreads, 0, launch_stream(s)>>>(
-                    o.incident_dof, o.incident_offset, o.incident_edge, o.incident_sign, o.incident_dofs, o.connection_count,
-                    o.conn_lower, o.conn_upper, o.conn_lower_node, o.conn_upper_node, o.conn_correction, o.conn_upper_weight,
-                    o.conn_area, o.reg_lower, o.reg_upper, o.reg_lower_node, o.reg_upper_node, o.reg_correction,
-                    o.reg_upper_weight, o.reg_area, gradient, s.active, out);
-        }
-        cuda_check(cudaGetLastError(), "launch allocation-free pressure operator");
+        apply_operator(s, p, out, orthogonal_only, !orthogonal_only && o.gradient_nodes ? noalloc_scratch(s) : nullptr);
     }
 }

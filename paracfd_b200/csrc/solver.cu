@@ -1330,9 +1330,7 @@ namespace pcfd
             if (!std::isfinite(rhs2) || rhs2 < 0) { result.relative_residual = std::numeric_limits<double>::infinity(); return result; }
             auto true_residual = [&]() {
                 launch_apply(s, x, s.t, true);
-                cuda_check(cudaMemcpyAsync(s.r, b, size_t(s.S) * sizeof(double), cudaMemcpyDeviceToDevice, s.stream), "copy rhs");
-                vec_subtract(s, s.r, s.t);
-                return device_dot(s, s.r, s.r);
+                return vec_residual_dot(s, b, s.t, s.r);
             };
             double residual2;
             if (warm) residual2 = true_residual();
@@ -1411,9 +1409,7 @@ namespace pcfd
             if (!std::isfinite(rhs2) || rhs2 < 0) { result.relative_residual = std::numeric_limits<double>::infinity(); return result; }
             auto true_residual = [&]() {
                 launch_apply(s, x, s.Ad, false);
-                cuda_check(cudaMemcpyAsync(s.defect, b, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s.stream), "copy rhs");
-                vec_subtract(s, s.defect, s.Ad);
-                return device_dot(s, s.defect, s.defect);
+                return vec_residual_dot(s, b, s.Ad, s.defect);
             };
             auto ru = [&](int c) { return s.recycle_u.p + size_t(c) * ld; };
             auto rcv = [&](int c) { return s.recycle_c.p + size_t(c) * ld; };
@@ -1463,9 +1459,7 @@ namespace pcfd
                 {
                     vec_copy_active(s, s.defect, s.r);
                     launch_apply(s, s.correction, s.Ad, false);
-                    cuda_check(cudaMemcpyAsync(s.defect, b, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s.stream), "copy rhs");
-                    vec_subtract(s, s.defect, s.Ad);
-                    true_recycled2 = device_dot(s, s.defect, s.defect);
+                    true_recycled2 = vec_residual_dot(s, b, s.Ad, s.defect);
                     vec_axpy_active(s, s.r, s.defect, -1.0);
                     gap2 = device_dot(s, s.r, s.r);
                 }
@@ -1828,9 +1822,7 @@ namespace pcfd
             pcfd_solve_result result = solve_orthogonal(s, x, b, tolerance, budget, warm);
             if (!(rhs2 > 0) || !std::isfinite(rhs2)) return result;
             launch_apply(s, x, s.Ad, true);
-            cuda_check(cudaMemcpyAsync(s.defect, b, size_t(s.S) * sizeof(double), cudaMemcpyDeviceToDevice, s.stream), "copy rhs");
-            vec_subtract(s, s.defect, s.Ad);
-            result.relative_residual = std::sqrt(device_dot(s, s.defect, s.defect) / rhs2);
+            result.relative_residual = std::sqrt(vec_residual_dot(s, b, s.Ad, s.defect) / rhs2);
             result.converged = std::isfinite(result.relative_residual) && result.relative_residual <= tolerance;
             return result;
         }
