@@ -317,6 +317,7 @@ namespace pcfd
         template <class T> void d2h(System& s, T* dst, const T* src, size_t n)
         {
             require(dst != nullptr || n == 0, "null host buffer");
+            if (n && threaded_download(s, dst, src, n * sizeof(T))) return;
             if (n) cuda_check(cudaMemcpyAsync(dst, src, n * sizeof(T), cudaMemcpyDeviceToHost, s.stream), "device to host");
         }
         void sync(System& s) { cuda_check(cudaStreamSynchronize(s.stream), "synchronize"); }
