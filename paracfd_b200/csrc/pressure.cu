@@ -188,13 +188,13 @@ namespace pcfd
         }
 
         // Fluxes of the compact edges at each incident DOF (reference amr_pressure.cu:105-178), a thread per
-        // DOF: the two-point sum in the reference's per-DOF order, sign * coefficient * (p[lower] -
-        // p[upper]) evaluated as coefficient * (p[dof] - p[other]) (equal bit for bit: negating a
-        // difference or a product is exact), then with kCorrected the WLS affine-exact non-orthogonal
+        // DOF: with kPart & 1 the two-point sum in the reference's per-DOF order, sign * coefficient *
+        // (p[lower] - p[upper]) evaluated as coefficient * (p[dof] - p[other]) (equal bit for bit: negating
+        // a difference or a product is exact), with kPart & 2 the WLS affine-exact non-orthogonal
         // corrections, out += each sum.  Entries have active endpoints only (build_operator drops the
         // others) and hold everything but the values, so a row is three loads deep; as two launches
         // over edge-indexed arrays the sums took 30 us against 21 for the 297 k DOFs of a 5.1 M-cell grid.
-        template <bool kCorrected>
+        template <int kPart>
         __global__ void __launch_bounds__(kRowThreads) irregular_gather_kernel(const int* __restrict__ incident_dof,
             const int* __restrict__ incident_offset, const int* __restrict__ incident_other, const double* __restrict__ incident_coefficient,
             const int2* __restrict__ incident_nodes, const double* __restrict__ incident_correction, int incident_dofs,
@@ -210,8 +210,8 @@ namespace pcfd
 #pragma unroll 2
             for (int q = q0; q < q1; ++q)
             {
-                two_point += incident_coefficient[q] * (centre - p[incident_other[q]]);
-                if (kCorrected)
+                if (kPart & 1) two_point += incident_coefficient[q] * (centre - p[incident_other[q]]);
+                if (kPart & 2)
                 {
                     const int2 n = incident_nodes[q];
                     const double* c = incident_correction + 5 * int64_t(q);
@@ -219,7 +219,7 @@ namespace pcfd
                     correction += n.x >= 0 ? -signed_area * face_derivative(gradient, n.x, n.y, corr, upper_weight) : 0.0;
                 }
             }
-            out[dof] = kCorrected ? (before + two_point) + correction : before + two_point;
+            out[dof] = kPart == 3 ? (before + two_point) + correction : before + (kPart == 1 ? two_point : correction);
         }
 
         __global__ void gauge_apply_kernel(const int* dof, const double* coefficient, int count, const double* p, double* out)
@@ -267,13 +267,18 @@ namespace pcfd
             else if (corrected)
                 reconstruct_gradient_kernel<<<blocks_for(o.gradient_nodes, kRowThreads), kRowThreads, 0, launch_stream(s)>>>(
                     o.grad_dof, o.grad_offset, o.grad_neighbour, o.grad_weight, p, gradient, o.gradient_nodes);
+            auto edges = [&](auto* kernel) {
+                if (o.incident_dofs)
+                    launch_chained(s, kernel, unsigned(blocks_for(o.incident_dofs, kRowThreads)), kRowThreads, o.incident_dof,
+                                   o.incident_offset, o.incident_other, o.incident_coefficient, o.incident_nodes, o.incident_correction,
+                                   o.incident_dofs, p, gradient, out);
+            };
+            // gauges (closed components of the flow region) are added between the two sums of a row
+            const bool together = corrected && !o.gauges;
+            edges(together ? irregular_gather_kernel<3> : irregular_gather_kernel<1>);
             if (o.gauges)
                 gauge_apply_kernel<<<blocks_for(o.gauges), kThreads, 0, launch_stream(s)>>>(o.gauge_dof, o.gauge_coefficient, o.gauges, p, out);
-            if (o.incident_dofs)
-                launch_chained(s, corrected ? irregular_gather_kernel<true> : irregular_gather_kernel<false>,
-                               unsigned(blocks_for(o.incident_dofs, kRowThreads)), kRowThreads, o.incident_dof, o.incident_offset,
-                               o.incident_other, o.incident_coefficient, o.incident_nodes, o.incident_correction, o.incident_dofs, p,
-                               gradient, out);
+            if (corrected && !together) edges(irregular_gather_kernel<2>);
             cuda_check(cudaGetLastError(), "launch pressure operator");
         }
     }
