@@ -109,6 +109,8 @@ namespace pcfd
             for (int u = 0; u <= V; ++u) acc[u] = 0.0;
             const int count = Q.size(), ucount = U.size();
             const int lane = threadIdx.x & 31, quarter = lane >> 3;
+            chain_wait();
+            chain_release();
             if (kMode >= 0)
             {
                 if (threadIdx.x < kMaxSet) coefficient[threadIdx.x] = threadIdx.x < count ? h[threadIdx.x] : 0.0;
@@ -276,6 +278,8 @@ namespace pcfd
             const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
             const int first = V * (warp / kShare), share = warp % kShare;
             const bool norms = warp < kShare;
+            chain_wait();
+            chain_release();
             for (int64_t item = blockIdx.x; item < range.items; item += gridDim.x)
             {
                 const int64_t base = range.base(item);
@@ -344,6 +348,8 @@ namespace pcfd
             __shared__ double shared[8];
             __shared__ bool last;
             const int j = blockIdx.x;
+            chain_wait();
+            chain_release();
             const bool used = j < count || (j >= kMaxSet && j < kMaxSet + count) || j >= 2 * kMaxSet;
             double v = 0.0;
             if (used)
@@ -366,28 +372,27 @@ namespace pcfd
             __shared__ double sum[kDcgsStride];
             if (threadIdx.x < 2 * kMaxSet + 3) sum[threadIdx.x] = __ldcg(total + threadIdx.x);
             __syncthreads();
-            if (threadIdx.x != 0) return;
-            *ticket = 0u;
+            if (threadIdx.x >= kMaxSet) return;      // the first warp: the sums in every lane, a coefficient per lane
+            const int l = threadIdx.x;
             double ss = 0.0, st = 0.0, tt = 0.0;
-            for (int l = 0; l < count; ++l)
+            for (int i = 0; i < count; ++i)
             {
-                ss += sum[l] * sum[l];
-                st += sum[l] * sum[kMaxSet + l];
-                tt += sum[kMaxSet + l] * sum[kMaxSet + l];
+                ss += sum[i] * sum[i];
+                st += sum[i] * sum[kMaxSet + i];
+                tt += sum[kMaxSet + i] * sum[kMaxSet + i];
             }
             const double vv = sum[2 * kMaxSet], vw = sum[2 * kMaxSet + 1], ww = sum[2 * kMaxSet + 2];
             const double r2 = vv - ss, r = r2 > 0.0 ? sqrt(r2) : 0.0;
             const double c = r > 0.0 ? (vw - st) / r : 0.0;
             const double rho2 = ww - tt - c * c, rho = rho2 > 0.0 ? sqrt(rho2) : 0.0;
             const double inv_r = r > 0.0 ? 1.0 / r : 0.0, c_r = c * inv_r;
-            for (int l = 0; l < kMaxSet; ++l)
-            {
-                const bool in = l < count;
-                out[l] = in ? sum[l] : 0.0;
-                out[kMaxSet + l] = in ? sum[kMaxSet + l] : 0.0;
-                out[2 * kMaxSet + l] = in ? sum[l] * inv_r : 0.0;
-                out[3 * kMaxSet + l] = in ? sum[kMaxSet + l] - c_r * sum[l] : 0.0;
-            }
+            const bool in = l < count;
+            out[l] = in ? sum[l] : 0.0;
+            out[kMaxSet + l] = in ? sum[kMaxSet + l] : 0.0;
+            out[2 * kMaxSet + l] = in ? sum[l] * inv_r : 0.0;
+            out[3 * kMaxSet + l] = in ? sum[kMaxSet + l] - c_r * sum[l] : 0.0;
+            if (l != 0) return;
+            *ticket = 0u;
             double* sc = out + 4 * kMaxSet;
             sc[0] = vv; sc[1] = vw; sc[2] = ww; sc[3] = r; sc[4] = c; sc[5] = rho; sc[6] = inv_r; sc[7] = c_r;
             sc[8] = rho > 0.0 ? 1.0 / rho : 0.0;
@@ -403,6 +408,7 @@ namespace pcfd
             double* __restrict__ vv, const double* __restrict__ w, double* __restrict__ next, const uint8_t* __restrict__ active, Sweep range)
         {
             __shared__ double cv[kMaxSet], cw[kMaxSet];
+            chain_wait();
             if (threadIdx.x < kMaxSet)
             {
                 cv[threadIdx.x] = coefficient[2 * kMaxSet + threadIdx.x];
@@ -485,7 +491,7 @@ namespace pcfd
             int grid = 0;
             auto go = [&](auto kernel) {
                 grid = block_grid(kernel);
-                kernel<<<grid, kThreadsBlock, 0, launch_stream(s)>>>(Q, h, w, U, sign, y, s.active, sweep_range(s), s.block_partial);
+                launch_chained(s, kernel, unsigned(grid), kThreadsBlock, Q, h, w, U, sign, y, s.active, sweep_range(s), s.block_partial);
             };
             if (m <= 4) go(block_kernel<1, kMode>);
             else if (m <= 8) go(block_kernel<2, kMode>);
@@ -557,7 +563,7 @@ namespace pcfd
         int grid = 0;
         auto dot = [&](auto kernel) {
             grid = block_grid(kernel);
-            kernel<<<grid, kThreadsBlock, 0, launch_stream(s)>>>(Q, v, w, s.active, range, s.dcgs_partial);
+            launch_chained(s, kernel, unsigned(grid), kThreadsBlock, Q, v, w, s.active, range, s.dcgs_partial);
         };
         // the fewest running sums that hold the m vectors (kMaxSet = 32)
         if (m <= 2) dot(dcgs_dot_kernel<2, 1>);
@@ -565,10 +571,9 @@ namespace pcfd
         else if (m <= 8) dot(dcgs_dot_kernel<4, 2>);
         else if (m <= 16) dot(dcgs_dot_kernel<8, 2>);
         else dot(dcgs_dot_kernel<8, 4>);
-        dcgs_final_kernel<<<2 * kMaxSet + 3, 256, 0, launch_stream(s)>>>(s.dcgs_partial, grid, m, s.dcgs_total, s.dcgs_ticket,
-                                                                       coefficient);
-        dcgs_update_kernel<<<block_grid(dcgs_update_kernel), kThreadsBlock, 0, launch_stream(s)>>>(Q, coefficient, v, w, next, s.active,
-                                                                                                  range);
+        launch_chained(s, dcgs_final_kernel, 2u * kMaxSet + 3, 256u, s.dcgs_partial, grid, m, s.dcgs_total, s.dcgs_ticket, coefficient);
+        launch_chained(s, dcgs_update_kernel, unsigned(block_grid(dcgs_update_kernel)), kThreadsBlock, Q, coefficient, v, w, next, s.active,
+                       range);
     }
 
     void block_combine(System& s, const VecSet& Z, const Coefficients& c, double* y, bool accumulate)

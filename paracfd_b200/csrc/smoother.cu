@@ -308,7 +308,12 @@ namespace pcfd
             int64_t b = blockIdx.x;
             if (b >= bricks) return;
             const int64_t G = gridDim.x;
-            Ticket cur = load_ticket(v, b);
+            Ticket cur = load_ticket(v, b);      // static: ahead of the wait for what the previous launch wrote
+            if (kMode != 2)
+            {
+                chain_wait();
+                chain_release();
+            }
             issue_brick<T, kWithR>(cur, z, r, v.code, tile[0], rbuf[0], cbuf[0]);
             if (kProlong == 2) issue_stage_values<TC>(cur, e, ebuf[0]);
             copy_commit();
@@ -464,6 +469,7 @@ namespace pcfd
                                            const uint8_t* __restrict__ active, const double* __restrict__ r,
                                            T* __restrict__ z, T* __restrict__ r_copy, int64_t structured, int64_t n, double omega)
         {
+            chain_release();
             const int64_t q0 = 4 * (int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
             if (q0 >= n) return;
             if (q0 + 4 > n)
@@ -556,6 +562,7 @@ namespace pcfd
             __shared__ __align__(16) double rtile[2][kTileSize];
             __shared__ __align__(16) T tile[kTileSize];
             __shared__ __align__(16) uint8_t cbuf[kCSize];
+            chain_release();
             int64_t b = blockIdx.x;
             if (b >= bricks) return;
             const int64_t G = gridDim.x;
@@ -729,6 +736,8 @@ namespace pcfd
             const int begin = low.y, end = high.y + (high.w >> 8);
             const int a = row.x, edges = here ? row.w >> 8 : 0, gauges = (row.w >> 2) & 63;
             const bool on = row.w & 1, incident = row.w & 2;
+            chain_wait();
+            chain_release();
             // the prolonged iterate at DOF q with map index c (active DOFs only)
             auto value = [&](int q, int c) {
                 if (kProlong == 3)
@@ -798,6 +807,7 @@ namespace pcfd
         __global__ void gather_base_kernel(int cells, const int* __restrict__ offset, const int* __restrict__ entry,
                                            const double* __restrict__ partial, const double* __restrict__ deferred, TC* __restrict__ rhs)
         {
+            chain_wait();
             const int c = blockIdx.x * blockDim.x + threadIdx.x;
             if (c >= cells) return;
             double sum = 0.0;
@@ -1121,10 +1131,9 @@ namespace pcfd
             FineSmoother& f = s.fine;
             if (!f.deferred_count) return;
             require(kProlong != 2 || f.map_attached, "deferred rows: composite map indices not attached");
-            finish_deferred_kernel<kMode, T, TO, TC, kProlong, TR>
-                <<<blocks_for(f.deferred_count, kFinishThreads), kFinishThreads, 0, launch_stream(s)>>>(
-                    deferred_view(s, omega), f.deferred_count, s.structured, e, kProlong == 3 ? scale : s.mg_prolong_scale, z, r, t, out,
-                    f.deferred_residual, r_copy);
+            launch_chained(s, finish_deferred_kernel<kMode, T, TO, TC, kProlong, TR>, unsigned(blocks_for(f.deferred_count, kFinishThreads)),
+                           kFinishThreads, deferred_view(s, omega), f.deferred_count, s.structured, e,
+                           kProlong == 3 ? scale : s.mg_prolong_scale, z, r, t, out, f.deferred_residual, r_copy);
         }
 
         // Persistent grid of a pipeline kernel: the system's CTAs per SM (autotuned), capped by the
@@ -1168,8 +1177,13 @@ namespace pcfd
             const bool cheb = slot >= 0 && w.chebyshev;
             const T* damping = cheb ? w.chebyshev + size_t(slot) * s.fine.cheb_stride : w.damping;
             const double omega = cheb ? s.fine.cheb_omega[slot] : 2.0 / 3.0;
-            brick_pipe_kernel<0, T, TO, TC, kProlong><<<pipe_grid<0, T>(s), 256, 0, launch_stream(s)>>>(
-                view(s), s.active_bricks, z, r, out, w.t, e, nullptr, damping);
+            // the prolongation's sweep follows a graph launch
+            if (kProlong)
+                brick_pipe_kernel<0, T, TO, TC, kProlong><<<pipe_grid<0, T>(s), 256, 0, launch_stream(s)>>>(
+                    view(s), s.active_bricks, z, r, out, w.t, e, nullptr, damping);
+            else
+                launch_chained(s, brick_pipe_kernel<0, T, TO, TC, kProlong>, unsigned(pipe_grid<0, T>(s)), 256u, view(s), s.active_bricks,
+                               z, r, out, w.t, e, nullptr, damping);
             finish<0, T, TO, TC, kProlong>(s, z, r, out, e, w.t, omega);
         }
         // Up to this many bricks the two pre-sweeps run as one launch (one preconditioner application on
@@ -1205,8 +1219,8 @@ namespace pcfd
         {
             FineSmoother& f = s.fine;
             FineBuffers<T> w(f);
-            brick_pipe_kernel<1, T, T, double, 0><<<pipe_grid<1, T>(s), 256, 0, launch_stream(s)>>>(
-                view(s), s.active_bricks, z, r, nullptr, w.t, nullptr, f.partial, w.damping);
+            launch_chained(s, brick_pipe_kernel<1, T, T, double, 0>, unsigned(pipe_grid<1, T>(s)), 256u, view(s), s.active_bricks, z, r,
+                           nullptr, w.t, nullptr, f.partial, w.damping);
             finish<1, T, T, double, 0>(s, z, r, nullptr, nullptr, w.t);
         }
     }
@@ -1229,8 +1243,8 @@ namespace pcfd
         MgLevel<TC>& base = levels.front();
         auto coarse = [&](auto* zz, auto* rr) {
             restrict_residual(s, zz, rr);
-            gather_base_kernel<TC><<<blocks_for(base.cells), kThreads, 0, launch_stream(s)>>>(
-                base.cells, f.gather_offset, f.gather_entry, f.partial, f.deferred_residual, base.rhs);
+            launch_chained(s, gather_base_kernel<TC>, unsigned(blocks_for(base.cells)), kThreads, base.cells, f.gather_offset, f.gather_entry,
+                           f.partial, f.deferred_residual, base.rhs);
             multigrid_levels(s, levels);
         };
         if (std::is_same<TC, float>::value && f.z32.n)
@@ -1258,6 +1272,7 @@ namespace pcfd
         __global__ void gather_first_kernel(int cells, const int* __restrict__ offset, const int* __restrict__ dof,
                                             const TR* __restrict__ residual, TC* __restrict__ rhs)
         {
+            chain_wait();
             const int c = blockIdx.x * blockDim.x + threadIdx.x;
             if (c >= cells) return;
             double sum = 0.0;
@@ -1272,6 +1287,7 @@ namespace pcfd
         __global__ void __launch_bounds__(256) gather_first_brick_kernel(int cells, const int* __restrict__ slot,
             const int* __restrict__ offset, const int* __restrict__ dof, const TR* __restrict__ residual, TC* __restrict__ rhs)
         {
+            chain_wait();
             const int c = blockIdx.x * blockDim.x + threadIdx.x;
             if (c >= cells) return;
             const int block = c & 63;
@@ -1295,11 +1311,11 @@ namespace pcfd
         void gather_first(System& s, const TR* residual, MgLevel<TC>& first)
         {
             if (s.first_stage_bricks)
-                gather_first_brick_kernel<TC, TR><<<blocks_for(first.cells), kThreads, 0, launch_stream(s)>>>(
-                    first.cells, s.active_brick_list, s.fine_restrict_offset, s.fine_restrict_dof, residual, first.rhs);
+                launch_chained(s, gather_first_brick_kernel<TC, TR>, unsigned(blocks_for(first.cells)), kThreads, first.cells,
+                               s.active_brick_list, s.fine_restrict_offset, s.fine_restrict_dof, residual, first.rhs);
             else
-                gather_first_kernel<TC, TR><<<blocks_for(first.cells), kThreads, 0, launch_stream(s)>>>(
-                    first.cells, s.fine_restrict_offset, s.fine_restrict_dof, residual, first.rhs);
+                launch_chained(s, gather_first_kernel<TC, TR>, unsigned(blocks_for(first.cells)), kThreads, first.cells,
+                               s.fine_restrict_offset, s.fine_restrict_dof, residual, first.rhs);
         }
 
         // residual of the pre-smoothed z, its gather into stage 1, the stage V-cycle, the weighted
@@ -1356,8 +1372,8 @@ namespace pcfd
             FineSmoother& f = s.fine;
             double* a = f.z.p;
             double* res = s.fine_residual.p;
-            brick_pipe_kernel<3, double, double, TC, 0><<<pipe_grid<3, double>(s), 256, 0, launch_stream(s)>>>(
-                view(s), s.active_bricks, z, r, res, f.t.p, nullptr, nullptr, f.damping.p);
+            launch_chained(s, brick_pipe_kernel<3, double, double, TC, 0>, unsigned(pipe_grid<3, double>(s)), 256u, view(s), s.active_bricks,
+                           z, r, res, f.t.p, nullptr, nullptr, f.damping.p);
             finish<2, double, double, TC, 0>(s, z, r, res, static_cast<const TC*>(nullptr), f.t.p);
             gather_first<TC, double>(s, res, first);
             composite_levels(s);
@@ -1375,8 +1391,8 @@ namespace pcfd
             FineSmoother& f = s.fine;
             float *a = f.z32.p, *b = f.z32b.p, *r32 = f.r32.p, *res = f.res32.p;
             pre_sweeps<float, float>(s, r, a, b, r32, true);
-            brick_pipe_kernel<3, float, float, float, 0><<<pipe_grid<3, float>(s), 256, 0, launch_stream(s)>>>(
-                view(s), s.active_bricks, b, r32, res, f.t32.p, nullptr, nullptr, f.damping32.p);
+            launch_chained(s, brick_pipe_kernel<3, float, float, float, 0>, unsigned(pipe_grid<3, float>(s)), 256u, view(s), s.active_bricks,
+                           b, r32, res, f.t32.p, nullptr, nullptr, f.damping32.p);
             finish<2, float, float, float, 0>(s, b, r32, res, static_cast<const float*>(nullptr), f.t32.p);
             gather_first<float, float>(s, res, first);
             composite_levels(s);
@@ -1414,7 +1430,7 @@ namespace pcfd
         else if (stage == 1)
         {
             restrict_residual<double>(s, z, r);
-            gather_base_kernel<double><<<blocks_for(base.cells), kThreads, 0, launch_stream(s)>>>(
+            launch_chained(s, gather_base_kernel<double>, unsigned(blocks_for(base.cells)), kThreads,
                 base.cells, f.gather_offset, f.gather_entry, f.partial, f.deferred_residual, base.rhs);
         }
         else if (stage == 2)
