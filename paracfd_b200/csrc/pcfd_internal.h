@@ -431,7 +431,8 @@ namespace pcfd
     void brick_apply(System& s, const double* p, double* out);   // code-byte structured operator
     void fine_preconditioner_stage(System& s, int stage, const double* r, double* z);
     template <class T> void fine_preconditioner(System& s, const double* r, double* z, std::vector<MgLevel<T>>& levels);
-    template <class T> void multigrid_levels(System& s, std::vector<MgLevel<T>>& levels);
+    // the levels below the fine one; whether the next launch may be chained to their last (launch_chained)
+    template <class T> bool multigrid_levels(System& s, std::vector<MgLevel<T>>& levels);
     void build_composite(System& s, const pcfd_topology& t);
     // smoothing steps of a level as (c1, c2): d = c1 d + c2 D^-1 (b - A x), x += d (solver.cu)
     std::vector<std::pair<double, double>> smoothing_steps(int chebyshev, int sweeps);
@@ -440,7 +441,7 @@ namespace pcfd
     void plan_tail(std::vector<MgLevel<float>>& levels, const std::vector<HostRows>& rows, int coarsest_sweeps, double omega, StageTail& tail);
     void launch_tail(System& s, MgLevel<double>& level, const StageTail& tail);
     void launch_tail(System& s, MgLevel<float>& level, const StageTail& tail);
-    void composite_levels(System& s);                 // V-cycle below the fine level, composite chain
+    bool composite_levels(System& s);                 // the same for the composite chain
     int64_t krylov_sweep_entries(const System& s);    // vector entries the Krylov block kernels sweep
     void composite_preconditioner(System& s, const double* r, double* z);   // smoother.cu
     void learned_preconditioner(System& s, const double* r, double* z, bool coarse);   // smoother.cu

@@ -808,6 +808,7 @@ namespace pcfd
                                            const double* __restrict__ partial, const double* __restrict__ deferred, TC* __restrict__ rhs)
         {
             chain_wait();
+            chain_release();
             const int c = blockIdx.x * blockDim.x + threadIdx.x;
             if (c >= cells) return;
             double sum = 0.0;
@@ -1168,17 +1169,16 @@ namespace pcfd
         };
 
         // one fine sweep z + w (r - A z) / D; slot >= 0 selects the w of that step of the
-        // Chebyshev-Richardson schedule (mg_fine_chebyshev), otherwise w = 2/3
+        // Chebyshev-Richardson schedule (mg_fine_chebyshev), otherwise w = 2/3; not chained after a graph
         template <class T, class TO, class TC, int kProlong>
-        void sweep(System& s, const T* z, const T* r, TO* out, const TC* e, int slot = -1)
+        void sweep(System& s, const T* z, const T* r, TO* out, const TC* e, int slot = -1, bool chained = true)
         {
             FineBuffers<T> w(s.fine);
             require(kProlong != 2 || s.fine.stage_neighbour.p, "mapped prolongation: stage-1 brick ranks not set");
             const bool cheb = slot >= 0 && w.chebyshev;
             const T* damping = cheb ? w.chebyshev + size_t(slot) * s.fine.cheb_stride : w.damping;
             const double omega = cheb ? s.fine.cheb_omega[slot] : 2.0 / 3.0;
-            // the prolongation's sweep follows a graph launch
-            if (kProlong)
+            if (!chained)
                 brick_pipe_kernel<0, T, TO, TC, kProlong><<<pipe_grid<0, T>(s), 256, 0, launch_stream(s)>>>(
                     view(s), s.active_bricks, z, r, out, w.t, e, nullptr, damping);
             else
@@ -1245,22 +1245,22 @@ namespace pcfd
             restrict_residual(s, zz, rr);
             launch_chained(s, gather_base_kernel<TC>, unsigned(blocks_for(base.cells)), kThreads, base.cells, f.gather_offset, f.gather_entry,
                            f.partial, f.deferred_residual, base.rhs);
-            multigrid_levels(s, levels);
+            return multigrid_levels(s, levels);
         };
         if (std::is_same<TC, float>::value && f.z32.n)
         {
             float *a = f.z32.p, *b = f.z32b.p, *r32 = f.r32.p;
             pre_sweeps<float, TC>(s, r, a, b, r32, false);
-            coarse(b, r32);
-            sweep<float, float, TC, 1>(s, b, r32, a, base.x.p);
+            const bool chained = coarse(b, r32);
+            sweep<float, float, TC, 1>(s, b, r32, a, base.x.p, -1, chained);
             sweep<float, double, TC, 0>(s, a, r32, z, nullptr);
         }
         else
         {
             double* a = f.z.p;
             pre_sweeps<double, TC>(s, r, a, z, nullptr, false);
-            coarse(z, r);
-            sweep<double, double, TC, 1>(s, z, r, a, base.x.p);
+            const bool chained = coarse(z, r);
+            sweep<double, double, TC, 1>(s, z, r, a, base.x.p, -1, chained);
             sweep<double, double, TC, 0>(s, a, r, z, nullptr);
         }
         cuda_check(cudaGetLastError(), "fused preconditioner");
@@ -1273,6 +1273,7 @@ namespace pcfd
                                             const TR* __restrict__ residual, TC* __restrict__ rhs)
         {
             chain_wait();
+            chain_release();
             const int c = blockIdx.x * blockDim.x + threadIdx.x;
             if (c >= cells) return;
             double sum = 0.0;
@@ -1288,6 +1289,7 @@ namespace pcfd
             const int* __restrict__ offset, const int* __restrict__ dof, const TR* __restrict__ residual, TC* __restrict__ rhs)
         {
             chain_wait();
+            chain_release();
             const int c = blockIdx.x * blockDim.x + threadIdx.x;
             if (c >= cells) return;
             const int block = c & 63;
@@ -1376,8 +1378,8 @@ namespace pcfd
                            z, r, res, f.t.p, nullptr, nullptr, f.damping.p);
             finish<2, double, double, TC, 0>(s, z, r, res, static_cast<const TC*>(nullptr), f.t.p);
             gather_first<TC, double>(s, res, first);
-            composite_levels(s);
-            sweep<double, double, TC, 2>(s, z, r, a, first.x.p, schedule ? 2 : -1);
+            const bool chained = composite_levels(s);
+            sweep<double, double, TC, 2>(s, z, r, a, first.x.p, schedule ? 2 : -1, chained);
             sweep<double, double, TC, 0>(s, a, r, z, nullptr, schedule ? 3 : -1);
             cuda_check(cudaGetLastError(), "composite preconditioner");
         }
@@ -1395,8 +1397,8 @@ namespace pcfd
                            b, r32, res, f.t32.p, nullptr, nullptr, f.damping32.p);
             finish<2, float, float, float, 0>(s, b, r32, res, static_cast<const float*>(nullptr), f.t32.p);
             gather_first<float, float>(s, res, first);
-            composite_levels(s);
-            sweep<float, float, float, 2>(s, b, r32, a, first.x.p, 2);
+            const bool chained = composite_levels(s);
+            sweep<float, float, float, 2>(s, b, r32, a, first.x.p, 2, chained);
             sweep<float, double, float, 0>(s, a, r32, z, nullptr, 3);
             cuda_check(cudaGetLastError(), "composite preconditioner");
         }
@@ -1439,7 +1441,7 @@ namespace pcfd
         }
         else
         {
-            sweep<double, double, double, 1>(s, z, r, a, base.x.p);
+            sweep<double, double, double, 1>(s, z, r, a, base.x.p, -1, false);
             sweep<double, double, double, 0>(s, a, r, z, nullptr);
         }
     }
