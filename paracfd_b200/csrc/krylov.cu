@@ -193,8 +193,10 @@ namespace pcfd
 
         // out[j] = sum over blocks of partial[b * kStride + j], one CTA per sum j: thread partials over
         // b = t, t + 256, ..., a warp tree, then the 8 warps in order.  In one CTA all the sums' loads
-        // queued behind each other: 12.8 us on average over the columns of a cycle.
-        __global__ void __launch_bounds__(256) block_final_kernel(const double* __restrict__ partial, int blocks, double* __restrict__ out)
+        // queued behind each other: 12.8 us on average over the columns of a cycle.  host: a second copy
+        // in pinned host memory, or null (dcgs_final_kernel).
+        __global__ void __launch_bounds__(256) block_final_kernel(const double* __restrict__ partial, int blocks, double* __restrict__ out,
+                                                                  double* __restrict__ host)
         {
             chain_wait();
             chain_release();
@@ -210,6 +212,7 @@ namespace pcfd
                 double t = 0.0;
                 for (int w = 0; w < 8; ++w) t += shared[w];
                 out[j] = t;
+                if (host) host[j] = t;
             }
         }
 
@@ -239,6 +242,7 @@ namespace pcfd
         __global__ void __launch_bounds__(256) scale_by_inverse_norm_kernel(double* __restrict__ dst, const double* __restrict__ src,
             const double* __restrict__ norm2, const uint8_t* __restrict__ active, Sweep range)
         {
+            chain_wait();
             const double a = 1.0 / sqrt(fmax(0.0, norm2[0]));
             for (int64_t item = blockIdx.x; item < range.items; item += gridDim.x)
             {
@@ -341,9 +345,12 @@ namespace pcfd
         // One CTA per sum j (grid 2 kMaxSet + 3): thread partials over blocks b = t, t + 256, ...,
         // a warp tree, then the 8 warps in order, into total[j].  The CTA that finishes last (a
         // ticket taken after a memory fence, no waiting) forms the coefficients and resets the
-        // ticket for the next launch.
+        // ticket for the next launch.  host: a second copy of out in pinned host memory, or null: written
+        // from here it is there when the column's event is, and no copy engine's turn lies between
+        // this column and the next (65 k cells: 76 us a column with the copy, 69 without).
         __global__ void __launch_bounds__(256) dcgs_final_kernel(const double* __restrict__ partial, int blocks, int count,
-                                                                 double* total, unsigned* ticket, double* __restrict__ out)
+                                                                 double* total, unsigned* ticket, double* __restrict__ out,
+                                                                 double* __restrict__ host)
         {
             __shared__ double shared[8];
             __shared__ bool last;
@@ -387,15 +394,19 @@ namespace pcfd
             const double rho2 = ww - tt - c * c, rho = rho2 > 0.0 ? sqrt(rho2) : 0.0;
             const double inv_r = r > 0.0 ? 1.0 / r : 0.0, c_r = c * inv_r;
             const bool in = l < count;
-            out[l] = in ? sum[l] : 0.0;
-            out[kMaxSet + l] = in ? sum[kMaxSet + l] : 0.0;
-            out[2 * kMaxSet + l] = in ? sum[l] * inv_r : 0.0;
-            out[3 * kMaxSet + l] = in ? sum[kMaxSet + l] - c_r * sum[l] : 0.0;
-            if (l != 0) return;
-            *ticket = 0u;
-            double* sc = out + 4 * kMaxSet;
-            sc[0] = vv; sc[1] = vw; sc[2] = ww; sc[3] = r; sc[4] = c; sc[5] = rho; sc[6] = inv_r; sc[7] = c_r;
-            sc[8] = rho > 0.0 ? 1.0 / rho : 0.0;
+            if (l == 0) *ticket = 0u;
+            const double scalars[9] = {vv, vw, ww, r, c, rho, inv_r, c_r, rho > 0.0 ? 1.0 / rho : 0.0};
+            auto store = [&](double* to) {
+                to[l] = in ? sum[l] : 0.0;
+                to[kMaxSet + l] = in ? sum[kMaxSet + l] : 0.0;
+                to[2 * kMaxSet + l] = in ? sum[l] * inv_r : 0.0;
+                to[3 * kMaxSet + l] = in ? sum[kMaxSet + l] - c_r * sum[l] : 0.0;
+#pragma unroll
+                for (int i = 0; i < 9; ++i)
+                    if (l == i) to[4 * kMaxSet + i] = scalars[i];
+            };
+            store(out);
+            if (host) store(host);
         }
 
         // Pass 2: v <- v / r - Q (s / r) in place, next = (w - (c / r) v_old - Q (t - (c / r) s)) / rho.
@@ -528,18 +539,18 @@ namespace pcfd
         block_grid(dcgs_update_kernel);
     }
 
-    void block_dot(System& s, const VecSet& Q, const double* w, double* out)
+    void block_dot(System& s, const VecSet& Q, const double* w, double* out, double* host)
     {
         require(Q.size() >= 0 && Q.size() <= kMaxSet, "block dot: too many vectors");
         require(aligned16(w), "block dot: vector not 16-byte aligned");
         require_aligned(Q, "block dot: vector not 16-byte aligned");
         const VecSet none(Q.stride);
         const int grid = launch_block<-1>(s, Q, nullptr, const_cast<double*>(w), none, 0.0, nullptr);
-        launch_chained(s, block_final_kernel, unsigned(Q.size() + 1), 256u, s.block_partial, grid, out);
+        launch_chained(s, block_final_kernel, unsigned(Q.size() + 1), 256u, s.block_partial, grid, out, host);
     }
 
     void block_update(System& s, const VecSet& Q, const double* h, double* w, const VecSet& U, double sign, double* y, int mode,
-                      double* out)
+                      double* out, double* host)
     {
         require(Q.size() <= kMaxSet && U.size() <= Q.size(), "block update: invalid vector sets");
         require(aligned16(w) && (!U.size() || aligned16(y)), "block update: vector not 16-byte aligned");
@@ -550,10 +561,11 @@ namespace pcfd
         else if (mode == 1) grid = launch_block<1>(s, Q, h, w, U, sign, y);
         else grid = launch_block<2>(s, Q, h, w, U, sign, y);
         if (mode >= 1)
-            launch_chained(s, block_final_kernel, unsigned((mode == 2 ? Q.size() : 0) + 1), 256u, s.block_partial, grid, out);
+            launch_chained(s, block_final_kernel, unsigned((mode == 2 ? Q.size() : 0) + 1), 256u, s.block_partial, grid, out,
+                           host);
     }
 
-    void dcgs_pass(System& s, const VecSet& Q, double* v, const double* w, double* next, double* coefficient)
+    void dcgs_pass(System& s, const VecSet& Q, double* v, const double* w, double* next, double* coefficient, double* host)
     {
         require(Q.size() <= kMaxSet, "delayed CGS2: too many vectors");
         require(aligned16(v) && aligned16(w) && aligned16(next), "delayed CGS2: vector not 16-byte aligned");
@@ -571,7 +583,8 @@ namespace pcfd
         else if (m <= 8) dot(dcgs_dot_kernel<4, 2>);
         else if (m <= 16) dot(dcgs_dot_kernel<8, 2>);
         else dot(dcgs_dot_kernel<8, 4>);
-        launch_chained(s, dcgs_final_kernel, 2u * kMaxSet + 3, 256u, s.dcgs_partial, grid, m, s.dcgs_total, s.dcgs_ticket, coefficient);
+        launch_chained(s, dcgs_final_kernel, 2u * kMaxSet + 3, 256u, s.dcgs_partial, grid, m, s.dcgs_total, s.dcgs_ticket, coefficient,
+                       host);
         launch_chained(s, dcgs_update_kernel, unsigned(block_grid(dcgs_update_kernel)), kThreadsBlock, Q, coefficient, v, w, next, s.active,
                        range);
     }
@@ -587,6 +600,6 @@ namespace pcfd
     void scale_by_inverse_norm(System& s, double* dst, const double* src, const double* norm2)
     {
         require(aligned16(dst) && aligned16(src), "scale: vector not 16-byte aligned");
-        scale_by_inverse_norm_kernel<<<4 * 148, 256, 0, launch_stream(s)>>>(dst, src, norm2, s.active, sweep_range(s));
+        launch_chained(s, scale_by_inverse_norm_kernel, 4u * 148, 256u, dst, src, norm2, s.active, sweep_range(s));
     }
 }

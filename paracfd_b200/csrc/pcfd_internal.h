@@ -286,7 +286,7 @@ namespace pcfd
         DBuf<double> dcgs_total;                // [2 kMaxSet + 4] the partials' sums
         DBuf<unsigned> dcgs_ticket;             // CTAs of the sum kernel done (0 between launches)
         double* pinned_dcgs = nullptr;          // pinned host copies of dcgs_result, two columns
-        cudaEvent_t dcgs_ready[2] = {};         // readback of column j has landed in slot j & 1
+        cudaEvent_t dcgs_ready[2] = {};         // column j's coefficients are in slot j & 1 of the pinned copies
         bool delayed_orthogonalisation = false; // pcfd_options.gmres_delayed
         double* pinned_block = nullptr;         // pinned host copy of block_result
         DBuf<double> dot_result;                // device scalars
@@ -472,15 +472,17 @@ namespace pcfd
     void vec_update_direction(System& s, const double* z, double* d, double beta);
 
     // ---- fused block vector kernels (krylov.cu); all active-masked, deterministic ----
-    void block_dot(System& s, const VecSet& Q, const double* w, double* out);   // out[0..|Q|) = Q^T w, out[|Q|] = w.w
+    // out[0..|Q|) = Q^T w, out[|Q|] = w.w; host: a copy of out in pinned host memory, or null
+    void block_dot(System& s, const VecSet& Q, const double* w, double* out, double* host = nullptr);
     // w -= Q h; y += sign * U h[0..|U|); mode 1: out[0] = w'.w'; mode 2: out = Q^T w' then w'.w'
     void block_update(System& s, const VecSet& Q, const double* h, double* w, const VecSet& U, double sign, double* y, int mode,
-                      double* out);
+                      double* out, double* host = nullptr);
     void block_combine(System& s, const VecSet& Z, const Coefficients& c, double* y, bool accumulate);   // y (+)= Z c
     void scale_by_inverse_norm(System& s, double* dst, const double* src, const double* norm2);        // dst = src / sqrt(n2)
     // delayed CGS2 column step: reorthogonalise v against Q in place and write the next basis vector
     // from w; coefficient[0..4*kMaxSet+9) as dcgs_final_kernel documents (krylov.cu)
-    void dcgs_pass(System& s, const VecSet& Q, double* v, const double* w, double* next, double* coefficient);
+    void dcgs_pass(System& s, const VecSet& Q, double* v, const double* w, double* next, double* coefficient,
+                   double* host = nullptr);
     // looks up the grid of every block kernel once (an occupancy query), before any stream capture
     void prime_block_grids();
     constexpr int kDcgsCoefficients = 4 * kMaxSet + 9;

@@ -1561,8 +1561,8 @@ namespace pcfd
                             }
                         return std::abs(gg[cols]);
                     };
-                    // Column col's work (preconditioner, operator, both passes, coefficient readback)
-                    // is enqueued as one unit.
+                    // Column col's work (preconditioner, operator, both passes, which leave the
+                    // coefficients in pinned host memory too) is enqueued as one unit.
                     const int k = s.recycle_count;
                     auto enqueue = [&](int col) {
                         double* v = s.gmres_v.p + size_t(col) * ld;
@@ -1571,10 +1571,8 @@ namespace pcfd
                         launch_apply(s, zc, s.Ad, false);
                         VecSet Q = recycle_set(s.recycle_c.p);
                         for (int row = 0; row < col; ++row) Q.push(s.gmres_v.p + size_t(row) * ld);
-                        dcgs_pass(s, Q, v, s.Ad, s.gmres_v.p + size_t(col + 1) * ld, s.dcgs_result);
-                        cuda_check(cudaMemcpyAsync(s.pinned_dcgs + size_t(col & 1) * kDcgsCoefficients, s.dcgs_result.p,
-                                                   size_t(kDcgsCoefficients) * sizeof(double), cudaMemcpyDeviceToHost, s.stream),
-                                   "coefficient readback");
+                        dcgs_pass(s, Q, v, s.Ad, s.gmres_v.p + size_t(col + 1) * ld, s.dcgs_result,
+                                  s.pinned_dcgs + size_t(col & 1) * kDcgsCoefficients);
                         cuda_check(cudaEventRecord(s.dcgs_ready[col & 1], s.stream), "coefficient event");
                     };
                     enqueue(0);
@@ -1635,7 +1633,7 @@ namespace pcfd
                     // Column col's work: CGS2 of w = A z against [C | V_0..V_col].  The matching z -= U h_C
                     // update is deferred: its coefficients are kept per column and applied once when
                     // the cycle's correction is formed (z only enters the solution through Z y).
-                    // Coefficients and readback alternate between two sets of three blocks.
+                    // Coefficients and their host copies alternate between two sets of three blocks.
                     const int k = s.recycle_count;
                     auto enqueue = [&](int col) {
                         double* v = s.gmres_v.p + size_t(col) * ld;
@@ -1647,12 +1645,11 @@ namespace pcfd
                         for (int row = 0; row <= col; ++row) Q.push(s.gmres_v.p + size_t(row) * ld);
                         const size_t set = size_t(col & 1) * 3 * kStride;
                         double *b1 = h1 + set, *b2 = b1 + kStride, *b3 = b2 + kStride;
-                        block_dot(s, Q, s.Ad, b1);
-                        block_update(s, Q, b1, s.Ad, none, -1.0, nullptr, 2, b2);
-                        block_update(s, Q, b2, s.Ad, none, -1.0, nullptr, 1, b3);
+                        double* host = s.pinned_block + set;
+                        block_dot(s, Q, s.Ad, b1, host);
+                        block_update(s, Q, b1, s.Ad, none, -1.0, nullptr, 2, b2, host + kStride);
+                        block_update(s, Q, b2, s.Ad, none, -1.0, nullptr, 1, b3, host + 2 * kStride);
                         scale_by_inverse_norm(s, s.gmres_v.p + size_t(col + 1) * ld, s.Ad, b3);
-                        cuda_check(cudaMemcpyAsync(s.pinned_block + set, b1, size_t(3) * kStride * sizeof(double), cudaMemcpyDeviceToHost,
-                                                   s.stream), "coefficient readback");
                         cuda_check(cudaEventRecord(s.dcgs_ready[col & 1], s.stream), "coefficient event");
                     };
                     enqueue(0);
