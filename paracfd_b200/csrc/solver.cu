@@ -1119,7 +1119,7 @@ namespace pcfd
         // Runs mg_level over `chain` through a CUDA graph captured on first use (the chain and its
         // buffers are fixed for the system's lifetime), or, where it is one cluster launch, as that,
         // chained to its neighbours (65 k cells: 33.1 against 39.1 us an application; the levels of
-        // larger grids launched one by one 840 -> 849 us on 16 M, 225 -> 258 for the reference cycle).
+        // larger grids launched one by one: 840 -> 849 us on 16 M).
         // Returns whether its last launch is a kernel that the next may be chained to.
         template <class T>
         bool run_captured(System& s, std::vector<MgLevel<T>*>& chain, const StageTail& tail, cudaGraphExec_t& exec, int64_t& nodes)
