@@ -19,9 +19,11 @@
 //     remainder iterations each waited for their own neighbour (2.0-2.5 k cycles a step of 512 rows);
 //   * matrix and iterate are kept as doubles: the sums are FP64, and converting every FP32 or FP16
 //     operand (16 per cycle and SM) costs more than the sums themselves.  The iterate's values
-//     are rounded to T as before, so the arithmetic is that of the per-launch kernels (solver.cu):
-//     FP64 row sums in CSR order, d = c1 d + c2 D^-1 (b - A x), x += d (damped Jacobi is c1 = 0,
-//     c2 = omega), the first step of a correction from x = 0 without the matrix.
+//     are rounded to T as before, so the arithmetic is that of the per-launch kernels (solver.cu), with
+//     each level's couplings as that level stores them (the coarsest's never in FP16): FP64 row
+//     sums in CSR order (a brick-structured first stage sums its faces first when it is launched
+//     alone), d = c1 d + c2 D^-1 (b - A x), x += d (damped Jacobi is c1 = 0, c2 = omega), the first
+//     step of a correction from x = 0 without the matrix.
 //
 // Which levels: the longest run of levels at the coarse end whose rows fit kTailRows and whose
 // slices fit the CTAs' shared memory.
@@ -420,8 +422,9 @@ namespace pcfd
             return double(T(weight));
         }
 
-        // the CTAs' images
-        template <class T> std::vector<unsigned char> images(const std::vector<HostRows>& rows, int first, int ranks, bool dense, bool half, const TailArgs<T>& a)
+        // the CTAs' images.  half_stages: FP16 couplings, on every level but the coarsest, whose sweeps need them
+        // to add up to the diagonal (a closed domain's coarsest operator is singular)
+        template <class T> std::vector<unsigned char> images(const std::vector<HostRows>& rows, int first, int ranks, bool dense, bool half_stages, const TailArgs<T>& a)
         {
             std::vector<unsigned char> out(size_t(ranks) * size_t(a.image), 0);
             auto put = [&](int rank, int offset, int64_t index, auto value) {
@@ -432,7 +435,7 @@ namespace pcfd
             {
                 const TailLevel& l = a.level[k];
                 const HostRows& h = rows[size_t(first + k)];
-                const bool coarsest = k + 1 == a.count, matrix = !coarsest || !dense;
+                const bool coarsest = k + 1 == a.count, matrix = !coarsest || !dense, half = half_stages && !coarsest;
                 for (int r0 = 0, rank = 0; r0 < h.cells; r0 += l.chunk, ++rank)
                 {
                     int extras = 0, members = 0;

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from oracle import port
-from paracfd_b200 import MG_CYCLE_COMPOSITE, MG_CYCLE_REFERENCE, MG_FP32, MG_FP64, BuiltTopology, CompositeSystem
+from paracfd_b200 import MG_CYCLE_COMPOSITE, MG_CYCLE_REFERENCE, MG_FP32, MG_FP64, BuiltTopology, CompositeSystem, capi
 from paracfd_b200.geometry import extruded_wing, naca4_section, rotate_section
 
 pytestmark = pytest.mark.gpu
@@ -81,3 +81,26 @@ def test_solves_with_finer_levels_outside_the_launch(gpu, cycle, precision):
     built.close()
     assert got["converged"] and residual <= 1.01e-8, (got, residual)
     assert got["iterations"] <= want["iterations"] + 1, (got, want)
+
+
+STAGE_SMOOTH = 2                      # PCFD_PROFILE_STAGE_SMOOTH
+
+
+@pytest.mark.parametrize("fp16", [0, 1])
+def test_coarsest_level_without_inverse_keeps_its_precision(gpu, fp16):
+    """Without an outlet the coarsest operator is singular: no inverse, and its couplings stay FP32
+    also with FP16 stages (rounded to FP16 they would not add up to the diagonal, here by 2.4e-4 a
+    sweep).  The launch against the same cycle in launches of its own, which a profiled first stage
+    takes: equal to FP32 rounding, as above.  The cell size is no power of two, so FP16 rounds."""
+    built = grid(1, 1 / 12)
+    closed = capi.Topology.from_buffer_copy(built.topology)
+    closed.pressure_outlet_xmax = 0
+    act = built.active.astype(bool)
+    r = np.where(act, np.random.default_rng(5).standard_normal(built.storage_size), 0.0)
+    with CompositeSystem(closed, mg_cycle=MG_CYCLE_COMPOSITE, mg_precision=MG_FP32, mg_stage_fp16=fp16) as s:
+        together = s.precondition(r)
+        s.profile_begin(STAGE_SMOOTH, 64)
+        apart = s.precondition(r)
+        assert len(s.profile_end(64)) > 0
+    assert rel(together, apart, act) <= 1e-4
+    built.close()
