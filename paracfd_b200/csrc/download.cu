@@ -4,9 +4,11 @@
 // which also takes the page faults of a freshly allocated destination: 54 ms for the 310 MB of
 // velocity and pressure on the 16 M-cell grid (6 GB/s).  Here up to eight host threads take 1 MiB
 // pieces in turn: each stages its piece in pinned memory of its own (two pieces in flight) and
-// copies it on, so the faults and copies run side by side.  The pinned pieces belong to the system
-// and go with it.  Copies below kThreadedCopy, where starting threads costs more than it gives, and
-// copies into pinned memory stay plain.
+// copies it on, so the faults and copies run side by side.  Each thread has a stream of its own that
+// waits for what the caller's stream holds: the caller's may be cudaStreamPerThread, which in
+// another thread names another stream.  Pinned pieces and streams belong to the system and go with
+// it.  Copies below kThreadedCopy, where starting threads costs more than it gives, copies into
+// pinned memory and copies of a stream that is being captured stay plain.
 #include "pcfd_internal.h"
 
 #include <algorithm>
@@ -27,13 +29,18 @@ namespace pcfd
     {
         int threads = 0;
         char* pinned = nullptr;                         // [threads][2][kPiece]
+        cudaStream_t stream[kMostThreads] = {};
         cudaEvent_t ready[kMostThreads][2] = {};
+        cudaEvent_t produced = nullptr;                 // what the caller's stream held before the copies
         ~Download()
         {
-            if (pinned) cudaFreeHost(pinned);
+            for (cudaStream_t one : stream)
+                if (one) cudaStreamDestroy(one);
             for (auto& pair : ready)
                 for (cudaEvent_t e : pair)
                     if (e) cudaEventDestroy(e);
+            if (produced) cudaEventDestroy(produced);
+            if (pinned) cudaFreeHost(pinned);
         }
     };
 
@@ -52,7 +59,11 @@ namespace pcfd
                 d->threads = 1;
             }
             for (int t = 0; t < d->threads && d->threads > 1; ++t)
+            {
+                cuda_check(cudaStreamCreateWithFlags(&d->stream[t], cudaStreamNonBlocking), "download stream");
                 for (cudaEvent_t& e : d->ready[t]) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "download event");
+            }
+            if (d->threads > 1) cuda_check(cudaEventCreateWithFlags(&d->produced, cudaEventDisableTiming), "download event");
             s.download = std::move(d);
             return s.download->threads > 1;
         }
@@ -64,9 +75,16 @@ namespace pcfd
         cudaPointerAttributes where{};
         if (cudaPointerGetAttributes(&where, dst) != cudaSuccess) cudaGetLastError();
         else if (where.type != cudaMemoryTypeUnregistered) return false;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s.stream, &capture) != cudaSuccess) cudaGetLastError();
+        if (capture != cudaStreamCaptureStatusNone) return false;
         if (!staging(s)) return false;
         Download& d = *s.download;
         const size_t pieces = (bytes + kPiece - 1) / kPiece;
+        const int want = int(std::min<size_t>(size_t(d.threads), pieces));
+        // recorded by the calling thread, which is the one that enqueued the work
+        cuda_check(cudaEventRecord(d.produced, s.stream), "download event");
+        for (int t = 0; t < want; ++t) cuda_check(cudaStreamWaitEvent(d.stream[t], d.produced, 0), "download wait");
         std::atomic<size_t> next{0};
         std::atomic<int> failed{int(cudaSuccess)};
         auto work = [&](int t) {
@@ -82,8 +100,8 @@ namespace pcfd
                 held[b] = failed.load() ? pieces : next.fetch_add(1);
                 if (held[b] >= pieces) { held[b] = pieces; return; }
                 if (!check(cudaMemcpyAsync(stage + size_t(b) * kPiece, static_cast<const char*>(src) + held[b] * kPiece, size(held[b]),
-                                           cudaMemcpyDeviceToHost, s.stream)) ||
-                    !check(cudaEventRecord(d.ready[t][b], s.stream)))
+                                           cudaMemcpyDeviceToHost, d.stream[t])) ||
+                    !check(cudaEventRecord(d.ready[t][b], d.stream[t])))
                     held[b] = pieces;
             };
             start(0);
@@ -95,7 +113,6 @@ namespace pcfd
             }
         };
         std::vector<std::thread> helpers;
-        const int want = int(std::min<size_t>(size_t(d.threads), pieces));
         helpers.reserve(size_t(want));
         try
         {
@@ -108,7 +125,8 @@ namespace pcfd
         work(0);
         for (std::thread& h : helpers) h.join();
         // nothing may still write the pinned pieces or read the source after an error
-        if (failed.load()) cudaStreamSynchronize(s.stream);
+        if (failed.load())
+            for (int t = 0; t < want; ++t) cudaStreamSynchronize(d.stream[t]);
         cuda_check(cudaError_t(failed.load()), "device to host");
         return true;
     }
