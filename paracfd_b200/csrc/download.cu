@@ -46,6 +46,23 @@ namespace pcfd
 
     namespace
     {
+        // the system's device while this lives, then the thread's own again
+        struct OnDevice
+        {
+            int before = 0;
+            bool changed = false;
+            explicit OnDevice(int device)
+            {
+                cuda_check(cudaGetDevice(&before), "current device");
+                changed = before != device;
+                if (changed) cuda_check(cudaSetDevice(device), "set device");
+            }
+            ~OnDevice()
+            {
+                if (changed) cudaSetDevice(before);
+            }
+        };
+
         // the system's staging, made on its first large copy; false when the host has none to give
         bool staging(System& s)
         {
@@ -78,6 +95,8 @@ namespace pcfd
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s.stream, &capture) != cudaSuccess) cudaGetLastError();
         if (capture != cudaStreamCaptureStatusNone) return false;
+        // streams and events are made and recorded on the system's device, whichever this thread uses
+        const OnDevice on(s.device);
         if (!staging(s)) return false;
         Download& d = *s.download;
         const size_t pieces = (bytes + kPiece - 1) / kPiece;
@@ -92,7 +111,7 @@ namespace pcfd
                 if (e != cudaSuccess) failed.store(int(e));
                 return e == cudaSuccess;
             };
-            if (!check(cudaSetDevice(s.device))) return;
+            if (t > 0 && !check(cudaSetDevice(s.device))) return;
             char* const stage = d.pinned + size_t(t) * 2 * kPiece;
             size_t held[2] = {pieces, pieces};           // piece in flight per buffer
             auto size = [&](size_t p) { return std::min(kPiece, bytes - p * kPiece); };
