@@ -14,7 +14,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
-#include <system_error>
 #include <thread>
 
 namespace pcfd
@@ -69,18 +68,19 @@ namespace pcfd
             if (s.download) return s.download->threads > 1;
             auto d = std::make_shared<Download>();
             d->threads = int(std::min<unsigned>(kMostThreads, std::max(1u, std::thread::hardware_concurrency())));
-            if (d->threads > 1 && cudaMallocHost(&d->pinned, size_t(d->threads) * 2 * kPiece) != cudaSuccess)
+            bool made = d->threads > 1 && cudaMallocHost(&d->pinned, size_t(d->threads) * 2 * kPiece) == cudaSuccess &&
+                        cudaEventCreateWithFlags(&d->produced, cudaEventDisableTiming) == cudaSuccess;
+            for (int t = 0; t < d->threads && made; ++t)
+            {
+                made = cudaStreamCreateWithFlags(&d->stream[t], cudaStreamNonBlocking) == cudaSuccess;
+                for (cudaEvent_t& e : d->ready[t]) made = made && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+            }
+            if (!made)
             {
                 cudaGetLastError();
-                d->pinned = nullptr;
+                d = std::make_shared<Download>();
                 d->threads = 1;
             }
-            for (int t = 0; t < d->threads && d->threads > 1; ++t)
-            {
-                cuda_check(cudaStreamCreateWithFlags(&d->stream[t], cudaStreamNonBlocking), "download stream");
-                for (cudaEvent_t& e : d->ready[t]) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "download event");
-            }
-            if (d->threads > 1) cuda_check(cudaEventCreateWithFlags(&d->produced, cudaEventDisableTiming), "download event");
             s.download = std::move(d);
             return s.download->threads > 1;
         }
@@ -132,14 +132,14 @@ namespace pcfd
             }
         };
         std::vector<std::thread> helpers;
-        helpers.reserve(size_t(want));
         try
         {
+            helpers.reserve(size_t(want));
             for (int t = 1; t < want; ++t) helpers.emplace_back(work, t);
         }
-        catch (const std::system_error&)
+        catch (...)
         {
-            // fewer helpers: the threads there are take all pieces
+            // no memory or no thread for more: those there are take all pieces
         }
         work(0);
         for (std::thread& h : helpers) h.join();

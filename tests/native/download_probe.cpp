@@ -35,12 +35,20 @@ namespace
         int device = 0;
         Queue* queue = nullptr;      // recorded on; a wait runs all of its queue (later actions may run early)
     };
-    std::recursive_mutex lock;
     thread_local int current = 0;
     std::map<std::pair<int, std::thread::id>, Queue> per_thread;
     std::map<int, Queue> legacy;
     bool fail_device_memory = false;
     thread_local int allocations_left = -1;      // of this thread's operator new; < 0: no limit
+    // one call of the stand-in at a time; its own allocations do not count
+    struct Call
+    {
+        static std::recursive_mutex& lock() { static std::recursive_mutex one; return one; }
+        std::lock_guard<std::recursive_mutex> guard{lock()};
+        int left = allocations_left;
+        Call() { allocations_left = -1; }
+        ~Call() { allocations_left = left; }
+    };
 
     Queue& queue_of(cudaStream_t stream)
     {
@@ -73,6 +81,7 @@ extern "C"
     cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { a->type = cudaMemoryTypeUnregistered; return cudaSuccess; }
     cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned)
     {
+        const Call call;
         auto* q = new Queue;
         q->device = current;
         *s = reinterpret_cast<cudaStream_t>(q);
@@ -82,18 +91,19 @@ extern "C"
     cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = cudaStreamCaptureStatusNone; return cudaSuccess; }
     cudaError_t cudaStreamSynchronize(cudaStream_t s)
     {
-        std::lock_guard<std::recursive_mutex> guard(lock);
+        const Call call;
         queue_of(s).drain();
         return cudaSuccess;
     }
     cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t bytes, cudaMemcpyKind, cudaStream_t s)
     {
-        std::lock_guard<std::recursive_mutex> guard(lock);
+        const Call call;
         queue_of(s).pending.push_back([=] { std::memcpy(to, from, bytes); });
         return cudaSuccess;
     }
     cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned)
     {
+        const Call call;
         auto* event = new Event;
         event->device = current;
         *e = reinterpret_cast<cudaEvent_t>(event);
@@ -102,7 +112,7 @@ extern "C"
     cudaError_t cudaEventDestroy(cudaEvent_t e) { delete reinterpret_cast<Event*>(e); return cudaSuccess; }
     cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s)
     {
-        std::lock_guard<std::recursive_mutex> guard(lock);
+        const Call call;
         Queue& q = queue_of(s);
         Event& event = *reinterpret_cast<Event*>(e);
         if (event.device != q.device) return cudaErrorInvalidResourceHandle;
@@ -111,14 +121,14 @@ extern "C"
     }
     cudaError_t cudaEventSynchronize(cudaEvent_t e)
     {
-        std::lock_guard<std::recursive_mutex> guard(lock);
+        const Call call;
         Event& event = *reinterpret_cast<Event*>(e);
         if (event.queue) event.queue->drain();
         return cudaSuccess;
     }
     cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned)
     {
-        std::lock_guard<std::recursive_mutex> guard(lock);
+        const Call call;
         Queue* from = reinterpret_cast<Event*>(e)->queue;
         if (from) queue_of(s).pending.push_back([from] { from->drain(); });
         return cudaSuccess;

@@ -1,5 +1,6 @@
 """Large downloads and device buffers against a stand-in for the CUDA runtime (native/download_probe.cpp):
-which stream the copies follow and which device they run on, without a GPU."""
+which stream the copies follow, which device they run on and what a failed start of a helper leaves,
+without a GPU."""
 import os
 import subprocess
 
@@ -19,7 +20,7 @@ def probe(tmp_path_factory):
 
 
 @pytest.mark.skipif((os.cpu_count() or 1) < 2, reason="one host thread: downloads stay plain")
-@pytest.mark.parametrize("check", ["per-thread stream", "other device"])
+@pytest.mark.parametrize("check", ["per-thread stream", "other device", "failed thread start"])
 def test_threaded_download(probe, check):
     run = subprocess.run([probe, check], capture_output=True, text=True, timeout=60)
     assert run.returncode == 0, run.stdout + run.stderr
