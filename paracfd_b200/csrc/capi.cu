@@ -326,7 +326,7 @@ namespace pcfd
     // basis storage of the flexible GCRO/LGMRES solver
     void allocate_gcro(System& s)
     {
-        if (s.gmres_v.p) return;
+        if (s.recycle_c.p) return;   // the last of them
         s.gmres_v.alloc(size_t(System::gmres_restart + 1) * s.Sp);
         s.gmres_z.alloc(size_t(System::gmres_restart) * s.Sp);
         s.recycle_u.alloc(size_t(System::recycle_capacity) * s.Sp);

@@ -945,6 +945,7 @@ namespace pcfd
         void ensure_capacity(Learned& L, int samples)
         {
             if (samples <= L.capacity) return;
+            L.capacity = 0;          // until all of them are there
             const size_t n = size_t(samples);
             L.x0.alloc(n * 512 * 16); L.e0.alloc(n * 512 * 16); L.e1.alloc(n * 64 * 32); L.bt.alloc(n * 8 * 64);
             L.d1.alloc(n * 64 * 32); L.d0.alloc(n * 512 * 16);
@@ -959,11 +960,12 @@ namespace pcfd
         {
             if (!s.learned)
             {
-                s.learned = new Learned();
-                Learned& L = *s.learned;
+                auto fresh = std::make_unique<Learned>();
+                Learned& L = *fresh;
                 L.master.alloc(kParams); L.adam_m.alloc(kParams); L.adam_v.alloc(kParams); L.grad.alloc(kParams);
                 L.head.alloc(kHead); L.wf.alloc(kWeights); L.wt.alloc(kWeights);
                 L.scalars.alloc(4); L.error.alloc(1);
+                s.learned = fresh.release();
             }
             return *s.learned;
         }
@@ -1340,6 +1342,7 @@ namespace pcfd
         }
         if (L.eval_x.n < hx.size())
         {
+            L.eval_x.release();      // the last to be allocated: its size stands for all three
             L.eval_mask.alloc(hm.size(), false);
             L.eval_target.alloc(hx.size(), false);
             L.eval_x.alloc(hx.size(), false);

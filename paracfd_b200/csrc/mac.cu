@@ -716,6 +716,7 @@ namespace pcfd
         DBuf<float4> foot;                      // [3 faces] forward pass -> correction (Feet)
         DBuf<float2> range;
         DBuf<unsigned int> maximum;
+        bool extended = false;                  // ext_source, ext_slow and the buffers above are complete
         bool has_links = false;
     };
 
@@ -754,6 +755,7 @@ namespace pcfd
                 if (!list) st.ext_slow.alloc(size_t(st.slow_count), false);
                 list = st.ext_slow.p;
             }
+            st.extended = true;
         }
         void extend(System& s, const Faces& f)
         {
@@ -800,13 +802,14 @@ namespace pcfd
     void mac_set_links(System& s, const uint8_t* const host[3])
     {
         MacState& st = mac_state(s);
+        st.has_links = false;                   // until everything below is there
         for (int c = 0; c < 3; ++c)
         {
             st.links[c].upload(std::vector<uint8_t>(host[c], host[c] + s.faces));
             if (!st.forward[c].n) st.forward[c].alloc(size_t(s.faces));
         }
         if (!st.nut.n) st.nut.alloc(size_t(s.S));
-        if (!st.ext.n)
+        if (!st.extended)
         {
             st.foot.alloc(size_t(s.faces) * 3, false);
             st.range.alloc(size_t(s.faces) * 3, false);

@@ -66,9 +66,11 @@ namespace pcfd
         void alloc(size_t count, bool zero = true)
         {
             release();
-            n = count;
             if (!count) return;
-            cuda_check(cudaMalloc(&p, count * sizeof(T)), "cudaMalloc");
+            void* fresh = nullptr;
+            cuda_check(cudaMalloc(&fresh, count * sizeof(T)), "cudaMalloc");
+            p = static_cast<T*>(fresh);
+            n = count;               // only now: callers test n for "is there"
             if (zero) cuda_check(cudaMemset(p, 0, count * sizeof(T)), "cudaMemset");
         }
         void upload(const std::vector<T>& host)

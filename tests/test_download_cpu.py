@@ -24,3 +24,8 @@ def probe(tmp_path_factory):
 def test_threaded_download(probe, check):
     run = subprocess.run([probe, check], capture_output=True, text=True, timeout=60)
     assert run.returncode == 0, run.stdout + run.stderr
+
+
+def test_failed_allocation_leaves_no_size(probe):
+    run = subprocess.run([probe, "failed allocation"], capture_output=True, text=True, timeout=60)
+    assert run.returncode == 0, run.stdout + run.stderr
