@@ -390,7 +390,7 @@ namespace pcfd
         // Source of every node of every extended lattice: the index of a face of the component, -1 for
         // the nodes interpolated on another level (they are counted, and listed when `slow` is
         // given), -2 in covered bricks (never sampled).
-        __global__ void mac_source_kernel(MacView m, int64_t total, int* source, int* slow, int* count)
+        __global__ void mac_source_kernel(MacView m, int64_t total, int* source, int64_t* slow, int* count)
         {
             const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
             if (q >= total) return;
@@ -410,7 +410,7 @@ namespace pcfd
             if (from < 0)
             {
                 const int n = atomicAdd(count, 1);
-                if (slow) slow[n] = int(q);
+                if (slow) slow[n] = q;
             }
         }
         // Extended lattices of a field: copies, then the listed nodes interpolated on another level.
@@ -424,15 +424,15 @@ namespace pcfd
             const int from = source[q];
             if (from >= 0) ext[q] = f.c[int(q / per % 3)][from];
         }
-        __global__ void mac_extend_slow_kernel(MacView m, Faces f, int count, const int* __restrict__ slow, float* __restrict__ ext)
+        __global__ void mac_extend_slow_kernel(MacView m, Faces f, int count, const int64_t* __restrict__ slow, float* __restrict__ ext)
         {
             const int n = blockIdx.x * blockDim.x + threadIdx.x;
             if (n >= count) return;
-            const int q = slow[n];
+            const int64_t q = slow[n];
             const int bs = m.bs, per = ext_size(bs);
             const int64_t slot = q / (3 * per);
-            const int c = q / per % 3;
-            int local = q % per;
+            const int c = int(q / per % 3);
+            int local = int(q % per);
             const int nx = c == 0 ? bs + 3 : bs + 2, ny = c == 1 ? bs + 3 : bs + 2;
             const int i = local % nx - 1;
             local /= nx;
@@ -710,7 +710,8 @@ namespace pcfd
         DBuf<uint32_t> flags;
         DBuf<uint8_t> links[3];
         DBuf<float> forward[3], nut;
-        DBuf<int> ext_source, ext_slow;         // extended-lattice nodes: source faces, nodes interpolated on another level
+        DBuf<int> ext_source;                   // extended-lattice nodes: source faces
+        DBuf<int64_t> ext_slow;                 // the nodes interpolated on another level
         int slow_count = 0;
         DBuf<float> ext;                        // [B][3][ext_size] extended lattices of the field last extended
         DBuf<float4> foot;                      // [3 faces] forward pass -> correction (Feet)
@@ -738,13 +739,13 @@ namespace pcfd
         {
             MacState& st = mac_state(s);
             const int64_t total = ext_total(s);
-            require(total < (int64_t(1) << 31) && s.faces < (int64_t(1) << 31), "MAC momentum: grid too large");
+            require(s.faces < (int64_t(1) << 31), "MAC momentum: grid too large");   // a source is an int (1.9 billion cells)
             st.ext_source.alloc(size_t(total), false);
             st.ext.alloc(size_t(total));
             DBuf<int> count;
             count.alloc(1);
             const MacView m = mac_view(s);
-            int* list = nullptr;
+            int64_t* list = nullptr;
             for (int pass = 0; pass < 2; ++pass)
             {
                 cuda_check(cudaMemsetAsync(count.p, 0, sizeof(int), s.stream), "clear node count");
