@@ -21,9 +21,9 @@ F = np.float32
 U = 10.0
 
 
-def build(levels, brick_size):
+def build(levels, brick_size, base=0.125):
     vertices, triangles = extruded_wing(rotate_section(naca4_section(12, 48, 1.0), 4.0), -0.6, 0.6)
-    return BuiltTopology(vertices, triangles, (-1.0, -1.0, -1.0), (2.0, 1.0, 1.0), 0.125, levels, brick_size,
+    return BuiltTopology(vertices, triangles, (-1.0, -1.0, -1.0), (2.0, 1.0, 1.0), base, levels, brick_size,
                          wing_refinement_distance=0.3, surface_refinement_distance=0.1, wake_length=0.5, wake_radius=0.3)
 
 
@@ -185,6 +185,223 @@ def test_advection_matches_the_per_face_definition(gpu, levels, brick_size):
         moved = max(moved, abs(got - lattice.clamped(before, c, slot, ijk)))
         assert abs(got - want) <= 1e-5 * U, (levels, slot, c, ijk, got, want)
     assert moved > 1e-3 * U                                   # the step moved the field by 100 tolerances
+    for c in range(3):                                        # covered bricks' faces end as 0
+        assert not np.any(after[c][np.array(lattice.cov)])
+    built.close()
+
+
+class Faces(Lattice):
+    """The band update, the eddy viscosity and the diffusion of a face, from their definitions."""
+
+    def cell_point(self, s, ijk):
+        return [F(self.rec[s][a] + F(ijk[a] + 0.5) * self.h[self.level[s]]) for a in range(3)]
+
+    def stepped(self, c, axis, direction, s, ijk):
+        """(slot, face) one step along axis inside the level, or None."""
+        q, n = list(ijk), self.size(c)
+        q[axis] += direction
+        out = [a for a in range(3) if q[a] < 0 or q[a] >= n[a]]
+        if not out:
+            return s, q
+        nb = self.nb[s][2 * axis + (direction > 0)]
+        if len(out) > 1 or nb < 0 or self.cov[nb]:
+            return None
+        q[axis] -= direction * self.bs
+        return nb, q
+
+    def band(self, f, links, c, s, ijk, dt):
+        def minmod(a, b):
+            return 0.0 if a * b <= 0 else (a if abs(a) < abs(b) else b)
+
+        def opened(at, bit):
+            slot, q = at
+            return int(links[c][slot, q[2], q[1], q[0]]) >> bit & 1
+        here, p, h = (s, list(ijk)), self.point(c, s, ijk), float(self.h[self.level[s]])
+        current = low = high = self.clamped(f, c, s, ijk)
+        total = weights = 0.0
+        for axis in range(3):
+            velocity = self.sample(f, axis, s, p)[0]
+            up = -1 if velocity >= 0 else 1
+            bit, other = 2 * axis + (up > 0), 2 * axis + (up < 0)
+            first = self.stepped(c, axis, up, *here) if opened(here, bit) else None
+            if first is None:
+                continue
+            upstream = self.clamped(f, c, *first)
+            low, high = min(low, upstream), max(high, upstream)
+            weight = dt * abs(velocity) / h
+            delta = weight * (upstream - current)
+            second, down = self.stepped(c, axis, up, *first), self.stepped(c, axis, -up, *here)
+            if opened(here, other) and opened(first, bit) and second and down:
+                far, downstream = self.clamped(f, c, *second), self.clamped(f, c, *down)
+                low, high = min(low, downstream), max(high, downstream)
+                incoming = upstream + 0.5 * minmod(upstream - far, current - upstream)
+                delta = -weight * (current + 0.5 * minmod(current - upstream, downstream - current) - incoming)
+            total, weights = total + delta, weights + weight
+        return max(low, min(high, current + total / max(1.0, weights)))
+
+    def advected(self, f, links, c, s, ijk, dt):
+        def first(a, slot, q):
+            if int(links[a][slot, q[2], q[1], q[0]]) & 0x40:
+                return self.band(f, links, a, slot, q, dt)
+            return self.forward(f, a, slot, q, dt)[0]
+        if int(links[c][s, ijk[2], ijk[1], ijk[0]]) & 0x40:
+            return first(c, s, ijk)
+        value, low, high, back = self.forward(f, c, s, ijk, dt)
+        p, level = self.point(c, s, ijk), self.level[s]
+        foot = self.trace(f, s, p, -dt)
+        ahead, owner = self.locate(foot), self.locate(self.clamp(p))
+        if min(back, ahead, owner) < 0 or any(self.level[q] != level for q in (back, ahead, owner)):
+            return value
+
+        class Forward:                                    # the forward field, evaluated where it is read
+            def __init__(self, axis):
+                self.axis = axis
+
+            def __getitem__(self, q):
+                return first(self.axis, q[0], [q[3], q[2], q[1]])
+        again = self.sample([Forward(a) for a in range(3)], c, ahead, foot)[0]
+        return max(low, min(high, value + 0.5 * (self.clamped(f, c, s, ijk) - again)))
+
+    def eddy(self, f, s, ijk, cs):
+        h, centre = self.h[self.level[s]], self.cell_point(s, ijk)
+        g = np.empty((3, 3))
+        for c in range(3):
+            for axis in range(3):
+                lo, hi = list(centre), list(centre)
+                lo[axis], hi[axis] = F(lo[axis] - h), F(hi[axis] + h)
+                g[c, axis] = (self.sample(f, c, s, hi)[0] - self.sample(f, c, s, lo)[0]) / (2 * float(h))
+        strain = 0.5 * (g + g.T)
+        return (cs * float(h)) ** 2 * np.sqrt(2 * (strain ** 2).sum())
+
+    def cell(self, nut, s, ijk):
+        bs = self.bs
+
+        def clamped(slot, q):
+            i, j, k = (min(max(x, 0), bs - 1) for x in q)
+            return float(nut[slot, k, j, i])
+
+        def extended(slot, q):
+            terms = [((), 1.0)]
+            for x in q:
+                ends = ((0, 2.0), (1, -1.0)) if x < 0 else ((bs - 1, 2.0), (bs - 2, -1.0)) if x >= bs else ((x, 1.0),)
+                terms = [(t + (e,), w * v) for t, w in terms for e, v in ends]
+            return sum(w * clamped(slot, t) for t, w in terms)
+        out = [a for a in range(3) if ijk[a] < 0 or ijk[a] >= bs]
+        if not out:
+            return clamped(s, ijk)
+        if len(out) == 1:
+            a = out[0]
+            nb = self.nb[s][2 * a + (ijk[a] >= bs)]
+            if nb >= 0 and not self.cov[nb]:
+                q = list(ijk)
+                q[a] += bs if ijk[a] < 0 else -bs
+                return clamped(nb, q)
+        p = self.cell_point(s, ijk)
+        at = self.locate(p)
+        if at < 0:
+            return clamped(s, ijk)
+        x = [float(F((p[a] - self.rec[at][a]) / self.h[self.level[at]] - F(0.5))) for a in range(3)]
+        if self.level[at] == self.level[s]:
+            return clamped(at, [int(np.floor(v + 0.5)) for v in x])
+        i0, total = [int(np.floor(v)) for v in x], 0.0
+        for d in np.ndindex(2, 2, 2):
+            w = np.prod([x[a] - i0[a] if d[a] else 1.0 - (x[a] - i0[a]) for a in range(3)])
+            total += w * extended(at, [i0[a] + d[a] for a in range(3)])
+        return total
+
+    def diffused(self, f, links, nut, c, s, ijk, nu, dt):
+        link, current, viscosity, laplacian = int(links[c][s, ijk[2], ijk[1], ijk[0]]), self.clamped(f, c, s, ijk), nu, 0.0
+        for axis in range(3):
+            for direction in (-1, 1):
+                if not link & 0x40 or link >> (2 * axis + (direction > 0)) & 1:
+                    q = list(ijk)
+                    q[axis] += direction
+                    laplacian += self.node(f, c, s, q) - current
+        if not link & 0x40:
+            lower = list(ijk)
+            lower[c] -= 1
+            viscosity += 0.5 * (self.cell(nut, s, lower) + self.cell(nut, s, list(ijk)))
+        return current + dt * viscosity * laplacian / float(self.h[self.level[s]]) ** 2
+
+
+def smooth_faces(lattice, bricks):
+    """A smooth flow of the node positions, the same on both copies of a shared face."""
+    bs, out = lattice.bs, []
+    for c in range(3):
+        f = np.empty((bricks, bs + (c == 2), bs + (c == 1), bs + (c == 0)), np.float32)
+        k, j, i = np.meshgrid(*[np.arange(n) for n in f.shape[1:]], indexing="ij")
+        for slot in range(bricks):
+            h = float(lattice.h[lattice.level[slot]])
+            x, y, z = (float(lattice.rec[slot][a]) + (q + (0.0 if a == c else 0.5)) * h for a, q in enumerate((i, j, k)))
+            f[slot] = U * ((c == 0) + 0.3 * np.sin(2.1 * x + 1.3 * y + c) * np.cos(1.7 * z - 0.9 * y + 0.5 * c))
+        out.append(f)
+    return out
+
+
+def band_links(faces, rng):
+    """Half of the faces in the band, with open directions at random; the others open."""
+    return [np.where(rng.random(f.shape) < 0.5, 0x40 | rng.integers(0, 64, f.shape), 0x3F).astype(np.uint8) for f in faces]
+
+
+def picked(lattice, rng, count):
+    """Faces of non-covered bricks, half of the indices on the brick's rim."""
+    kept = [q for q in range(len(lattice.cov)) if not lattice.cov[q]]
+    for _ in range(count):
+        slot, c = int(rng.choice(kept)), int(rng.integers(3))
+        yield slot, c, [int(rng.choice([0, n - 1])) if rng.random() < 0.5 else int(rng.integers(n)) for n in lattice.size(c)]
+
+
+@pytest.mark.parametrize("levels,brick_size", [(1, 8), (3, 8), (2, 4)])
+def test_band_faces_match_the_per_face_definition(gpu, levels, brick_size):
+    """Advection with half of the faces in the near-surface band: bounds as above."""
+    built = build(levels, brick_size)
+    lattice = Faces(built.topology, brick_size)
+    rng = np.random.default_rng(23 * levels + brick_size)
+    with CompositeSystem(built.topology) as s:
+        before = smooth_faces(lattice, s.bricks)
+        links = band_links(before, rng)
+        s.set_faces(*[f.ravel() for f in before])
+        s.set_mac_links(*[q.ravel() for q in links])
+        dt = float(F(0.5 * float(min(lattice.h)) / (1.4 * U)))
+        s.mac_advect(dt)
+        after = [f.reshape(b.shape) for f, b in zip(s.get_faces(), before)]
+    moved = 0.0
+    for slot, c, ijk in picked(lattice, rng, 100):
+        want, got = lattice.advected(before, links, c, slot, ijk, dt), float(after[c][slot, ijk[2], ijk[1], ijk[0]])
+        moved = max(moved, abs(got - lattice.clamped(before, c, slot, ijk)))
+        assert abs(got - want) <= 1e-5 * U, (levels, slot, c, ijk, got, want)
+    assert moved > 1e-3 * U
+    built.close()
+
+
+@pytest.mark.parametrize("levels,brick_size,base", [(1, 8, 0.125), (3, 8, 0.125), (2, 4, 0.125), (3, 8, 1 / 12)])
+def test_diffusion_matches_the_per_face_definition(gpu, levels, brick_size, base):
+    """Eddy viscosity of a cell and diffusion of a face, half of the faces in the band.  A velocity
+    gradient is the difference of two samples (4e-6 U each) over 2 h: nine of them leave |S| within
+    2e-5 U / h.  The Laplacian's seven values err by 4e-6 U each, times a factor of at most 0.2.  With
+    cells of 1/12 the sample points one cell off a centre miss the ghost nodes by a rounding."""
+    built = build(levels, brick_size, base)
+    lattice = Faces(built.topology, brick_size)
+    rng = np.random.default_rng(31 * levels + brick_size)
+    nu, cs = 0.2, 0.17
+    with CompositeSystem(built.topology) as s:
+        before = smooth_faces(lattice, s.bricks)
+        links = band_links(before, rng)
+        s.set_faces(*[f.ravel() for f in before])
+        s.set_mac_links(*[q.ravel() for q in links])
+        dt = float(F(0.15 * float(min(lattice.h)) ** 2 / nu))
+        s.mac_diffuse_smagorinsky(nu, cs, dt)
+        after = [f.reshape(b.shape) for f, b in zip(s.get_faces(), before)]
+        nut = s.mac_eddy_viscosity()[:s.bricks * brick_size ** 3].reshape(s.bricks, *[brick_size] * 3)
+    moved = 0.0
+    for slot, c, ijk in picked(lattice, rng, 100):
+        cell = [min(q, brick_size - 1) for q in ijk]
+        h = float(lattice.h[lattice.level[slot]])
+        assert abs(float(nut[slot, cell[2], cell[1], cell[0]]) - lattice.eddy(before, slot, cell, cs)) <= (cs * h) ** 2 * 2e-5 * U / h, (slot, cell)
+        want, got = lattice.diffused(before, links, nut, c, slot, ijk, nu, dt), float(after[c][slot, ijk[2], ijk[1], ijk[0]])
+        moved = max(moved, abs(got - lattice.clamped(before, c, slot, ijk)))
+        assert abs(got - want) <= 1e-5 * U, (levels, slot, c, ijk, got, want)
+    assert moved > 1e-3 * U
     for c in range(3):                                        # covered bricks' faces end as 0
         assert not np.any(after[c][np.array(lattice.cov)])
     built.close()
