@@ -96,7 +96,7 @@ namespace pcfd
         DBuf<double> incident_correction;       // [entries][5]
         // regular corrections
         DBuf<int> reg_lower, reg_upper, reg_lower_node, reg_upper_node;
-        DBuf<double> reg_coefficient, reg_correction, reg_upper_weight, reg_area, reg_delta;
+        DBuf<double> reg_correction, reg_upper_weight, reg_delta;
         // WLS gradient nodes
         int gradient_nodes = 0;
         DBuf<int> grad_dof, grad_offset, grad_neighbour;
@@ -375,6 +375,10 @@ namespace pcfd
     // its memory is visible), so nothing it reads or writes overlaps the previous kernel, and then
     // calls chain_release() so that the next kernel may be scheduled once all its CTAs run.
     // Without a programmatic predecessor both are no-ops.
+    // Two exceptions.  A kernel launched plainly may release at once and never wait: all before it
+    // is complete.  reconstruct_gradient_kernel runs beside such a kernel (brick_apply) before it waits,
+    // so it relies on everything ahead of THAT kernel being complete: the launch of
+    // brick_apply must stay a plain one.
     __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
     __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
     template <typename T> struct Exactly { using type = T; };   // keeps Params deduced from the kernel only

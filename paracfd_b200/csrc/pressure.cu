@@ -474,8 +474,7 @@ namespace pcfd
             rw[e] = rc.upper_gradient_weight[e]; ra[e] = rc.open_area[e]; rd[e] = rc.two_point_delta[e];
         }
         o.reg_lower.upload(rl); o.reg_upper.upload(ru); o.reg_lower_node.upload(rln); o.reg_upper_node.upload(run);
-        o.reg_coefficient.upload(rcoef); o.reg_correction.upload(rcorr); o.reg_upper_weight.upload(rw);
-        o.reg_area.upload(ra); o.reg_delta.upload(rd);
+        o.reg_correction.upload(rcorr); o.reg_upper_weight.upload(rw); o.reg_delta.upload(rd);
 
         // Deterministic incidence: (dof, edge, sign) sorted, reference amr_pressure.cu:774-813.
         struct Incident { int dof, edge; int8_t sign; };
@@ -496,6 +495,7 @@ namespace pcfd
         std::vector<int> idof, ioff, iother;
         std::vector<int2> inodes;
         std::vector<double> icoef, icorr;
+        iother.reserve(inc.size()); inodes.reserve(inc.size()); icoef.reserve(inc.size()); icorr.reserve(5 * inc.size());
         for (size_t q = 0; q < inc.size(); ++q)
         {
             if (q == 0 || inc[q].dof != inc[q - 1].dof) { idof.push_back(inc[q].dof); ioff.push_back(int(q)); }

@@ -1225,6 +1225,8 @@ namespace pcfd
         }
     }
 
+    // Launched plainly, never chained: the WLS gradient that starts beside it reads p and writes its
+    // scratch without a wait, so what produced p and what last read the scratch must be complete here.
     void brick_apply(System& s, const double* p, double* out)
     {
         brick_pipe_kernel<2, double, double, double, 0><<<pipe_grid<2, double>(s), 256, 0, launch_stream(s)>>>(
