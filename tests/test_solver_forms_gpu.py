@@ -130,7 +130,8 @@ def test_fine_level_of_a_large_grid(gpu, cycle):
 @pytest.mark.parametrize("restart,recycle", [(24, 3), (9, 1), (8, -1), (1, 2)])
 def test_krylov_column_counts(gpu, delayed, restart, recycle):
     """Every number of columns a pass over the basis can hold, from one to restart + recycled pairs,
-    over several cycles and a second solve that starts from recycled pairs."""
+    over several cycles and a second solve that starts from recycled pairs.  Delayed: the dot pass of
+    grids up to 16,384 bricks (the pass of larger ones below)."""
     built = grid(2, 1 / 16)
     act = built.active.astype(bool)
     oracle = port.PortSystem(built.topology)
@@ -146,6 +147,52 @@ def test_krylov_column_counts(gpu, delayed, restart, recycle):
                 assert got["iterations"] <= want["iterations"] + 1, (got, want)
     oracle.close()
     built.close()
+
+
+@pytest.fixture(scope="module")
+def large(gpu):
+    built = grid(2, 1 / 64)
+    act = built.active.astype(bool)
+    assert act.sum() > 16384 * 512          # above: the dot pass whose warps share an item's entries
+    yield built, act
+    built.close()
+
+
+def test_delayed_columns_of_a_large_grid(large):
+    """The dot pass in each of its groupings (up to 2, 4, 8, 16 and 23 vectors before a column) against
+    the three-pass form: after as many columns both have the minimiser over the same space.  The
+    sums' rounding, 1e-16 of a column, grows at each orthogonalisation by the column's length before
+    over after it, some 3 on average: at most 1e-8 of the solution after 24 columns, so 1e-7."""
+    built, act = large
+    columns, found = (1, 3, 4, 5, 6, 9, 10, 17, 18, 24), []
+    for delayed in (0, 1):
+        with CompositeSystem(built.topology, mg_cycle=MG_CYCLE_REFERENCE, gmres_recycle=-1, gmres_delayed=delayed) as s:
+            b = s.apply(np.where(act, np.random.default_rng(4).standard_normal(built.storage_size), 0.0))
+            solves = [s.solve(b, 1e-14, n) for n in columns]
+            found.append([x[act] for x, _ in solves])
+            assert [got["iterations"] for _, got in solves] == list(columns)
+    for n, want, got in zip(columns, *found):
+        assert np.abs(got - want).max() <= 1e-7 * np.abs(want).max(), n
+    assert len({x.tobytes() for x in found[1]}) == len(columns)       # every column moved the solution
+
+
+@pytest.mark.parametrize("restart,recycle", [(24, 3), (5, 2)])
+def test_delayed_solves_of_a_large_grid(large, restart, recycle):
+    """Two solves, the second from recycled pairs, to the true residual (the operator is checked above)
+    in the columns of the three-pass form: rounding moves the last column of a cycle at most."""
+    built, act = large
+    iterations = []
+    for delayed in (0, 1):
+        with CompositeSystem(built.topology, mg_cycle=MG_CYCLE_REFERENCE, gmres_restart=restart, gmres_recycle=recycle,
+                             gmres_delayed=delayed) as s:
+            for seed in (4, 5):
+                b = s.apply(np.where(act, np.random.default_rng(seed).standard_normal(built.storage_size), 0.0))
+                x, got = s.solve(b, 1e-9, 2000)
+                residual = np.linalg.norm((b - s.apply(x))[act]) / np.linalg.norm(b[act])
+                assert got["converged"] and residual <= 1.01e-9, (got, residual)
+                iterations.append(got["iterations"])
+    for want, got in zip(iterations[:2], iterations[2:]):
+        assert abs(want - got) <= 1 + want // restart, iterations
 
 
 @pytest.mark.parametrize("n", [2, 5, 149, 301])
