@@ -668,9 +668,11 @@ namespace pcfd
             grid = block_grid(kernel);
             launch_chained(s, kernel, unsigned(grid), kThreadsBlock, Q, v, w, s.active, range, s.dcgs_partial);
         };
-        // Above, the pass is a large part of a column (19 M entries: 309 -> 192 us for m <= 8); below, the
-        // groups give 1 % of a column on 65 k cells, 3 % on 1.1 M and 5 % on 4.2 M, and the sums keep the
-        // order of one warp per vector instead, whose rounding a run's fields carry.
+        // The groups are the faster form at every size measured: 1 % of a column on 65 k cells, 3 % on 1.1 M,
+        // 5 % on 4.2 M, 309 -> 192 us for m <= 8 on 19 M entries.  The line is no crossover.  Up to it the sums
+        // keep the order of one warp per vector, so that the fields of those runs keep their rounding
+        // (dcgs_dot_warp_kernel); above it the gain was taken, and the fields of a ten-step run on 16 M
+        // cells moved by 1e-6.
         constexpr int64_t kGroupedDotItems = 16384;
         if (range.items <= kGroupedDotItems)
         {

@@ -418,9 +418,10 @@ namespace pcfd
             }
         }
         // Extended lattices of a field: copies, then the listed nodes interpolated on another level.
-        // The copy is bound by memory (4 B source, 4 B value, 4 B store per node; 3 x 1100 nodes per
-        // 8^3 brick); the interpolation's 64 clamped reads per node run in a launch of their own, so
-        // no copying warp waits for them.
+        // The copy moves 12 B per node (source, value, store; 3 x 1100 nodes per 8^3 brick) in rows of 8 to 10
+        // values, bound by L1 and L2 sectors (64 and 49 %): 47 us for 8.2 M nodes.  The interpolation's
+        // 64 clamped reads per node (77 us for 0.56 M) run in a launch of their own, so no copying warp
+        // waits for them.
         __global__ void mac_extend_kernel(Faces f, int per, int64_t total, const int* __restrict__ source, float* __restrict__ ext)
         {
             const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -452,9 +453,10 @@ namespace pcfd
         };
 
         // Forward pass, and both characteristics of the correction: they need the same field and start
-        // from the same velocity, so each face is traced back and forth once.  Bound by instruction
-        // issue and L1 gathers (ten trilinear samples, four locations per face): 0.57 ms for the 4.3 M
-        // faces of a 1.3 M-cell grid on three levels.  With the samples on the extended lattices and the
+        // from the same velocity, so each face is traced back and forth once.  Bound by the latency of ten
+        // trilinear samples and four locations per face at two CTAs an SM (110 registers; 44 % of the SM's
+        // throughput, 23 % of L1's, 22 % of its warps): 0.57 ms for the 4.3 M faces of a 1.3 M-cell grid on
+        // three levels.  With the samples on the extended lattices and the
         // traces shared, a whole advection takes 1.0 instead of 19.8 ms there (correction 0.14,
         // extensions 0.2 ms).
         __global__ void __launch_bounds__(256) mac_forward_kernel(MacView m, Faces f, Links links, int64_t total, float dt, Out out, Feet feet)

@@ -338,9 +338,9 @@ namespace pcfd
                 // x-adjacent cells (2 (t & 3), j, k)
                 // and (2 (t & 3) + 1, j, k), j = t >> 5, k = t >> 2 & 7: the stencil of a pair is five
                 // two-value reads and two single ones where two separate cells take fourteen, and codes,
-                // right-hand sides and results move as pairs.  The kernel is bound by instruction issue
-                // (77 % of the issue slots at 262 instructions per thread and brick with separate cells), so
-                // those reads, and the index arithmetic per copy and store, are its time.  With rows 12
+                // right-hand sides and results move as pairs.  With separate cells instruction issue was the
+                // limit (77 % of the slots at 262 instructions per thread and brick); with pairs issue (63 %), L1
+                // (66 %) and the barrier per brick share the time (5.1 M cells, three CTAs an SM).  With rows 12
                 // and planes 120 tile entries apart the lanes served together (a half-warp in float, four
                 // planes of eight values; a quarter-warp in double, two planes) fall on disjoint
                 // shared-memory banks (the staged rhs and codes are padded per plane for the same
@@ -355,8 +355,8 @@ namespace pcfd
                 if (kMode == 2)
                 {
                     // The operator keeps one cell at a time, (t & 7, t >> 5, (t >> 3 & 3) + 4 q): it is bound by
-                    // bytes rather than issue, and the pairs' single FP64 reads share banks (16 M cells: 102
-                    // against 104 us alone, and 189 against 194 with the gradient beside it).
+                    // loads rather than issue (49 % of the slots), and the pairs' single FP64 reads share
+                    // banks (16 M cells: 102 against 104 us alone, and 189 against 194 with the gradient beside it).
 #pragma unroll
                     for (int q = 0; q < 2; ++q)
                     {
