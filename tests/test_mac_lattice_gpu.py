@@ -1,4 +1,5 @@
-"""MacCormack advection of the staggered faces against a plain per-face restatement.
+"""MacCormack advection, band faces, eddy viscosity and diffusion of the staggered faces against a
+plain per-face restatement.
 
 mac_advect samples every field on per-brick lattices with one ghost node and shares the two
 characteristics between its passes.  The restatement below evaluates randomly chosen faces one by

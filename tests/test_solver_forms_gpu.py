@@ -106,6 +106,64 @@ def test_operator_forms(gpu, levels, h, embedded, gauges, fragments):
     built.close()
 
 
+@pytest.mark.parametrize("embedded,gauges,fragments", [(0, 0, 0), (129, 5, 1)])
+def test_captured_operator(gpu, embedded, gauges, fragments):
+    """The allocation-free operator in a CUDA graph on the caller's stream, chained launches included:
+    replayed on new values, the bits of a direct call."""
+    import torch
+    built = grid(3, 1 / 8)
+    topology, active = split_connections(built, embedded, gauges, fragments) if gauges else (built.topology, built.active.astype(bool))
+    n, lib, stream, handle = topology.storage_size, capi.load(), torch.cuda.Stream(), C.c_void_p()
+    capi.check(lib.pcfd_system_create(C.byref(topology), C.byref(capi.Options(stream=stream.cuda_stream)), C.byref(handle)))
+    p, out, direct = (torch.zeros(n, dtype=torch.float64, device="cuda:0") for _ in range(3))
+
+    def apply(to):
+        capi.check(lib.pcfd_pressure_apply_device_noalloc(handle, C.c_void_p(p.data_ptr()), C.c_void_p(to.data_ptr()), 0))
+    torch.cuda.synchronize()
+    apply(direct)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        apply(out)
+    for seed in (1, 2):
+        p.copy_(torch.from_numpy(np.where(active, np.random.default_rng(seed).standard_normal(n), 0.0)))
+        torch.cuda.synchronize()
+        for _ in range(2):
+            graph.replay()
+        torch.cuda.synchronize()
+        apply(direct)
+        torch.cuda.synchronize()
+        assert np.abs(direct.cpu().numpy()[active]).max() > 0
+        assert torch.equal(out, direct)
+    del graph
+    lib.pcfd_system_destroy(handle)
+    built.close()
+
+
+@pytest.mark.parametrize("levels,h,embedded,gauges,fragments", [
+    (1, 1 / 16, 0, 3, 0),           # gauges on a grid without compact edges
+    (2, 1 / 16, 1000, 0, 7),        # DOFs behind the bricks
+    (2, 1 / 16, 129, 5, 1),         # all three kinds of deferred row
+])
+@pytest.mark.parametrize("cycle", [MG_CYCLE_REFERENCE, MG_CYCLE_COMPOSITE])
+def test_fine_level_forms(gpu, cycle, levels, h, embedded, gauges, fragments):
+    """Deferred rows of embedded edges, gauges and DOFs behind the bricks in every fine-level pass, twice:
+    the second application finds the buffers as the first left them."""
+    built = grid(levels, h)
+    topology, active = split_connections(built, embedded, gauges, fragments)
+    n = topology.storage_size
+    oracle = port.PortSystem(topology)
+    if cycle == MG_CYCLE_COMPOSITE:
+        oracle.set_composite(6, 30, 10)
+    for precision, bound in ((MG_FP64, 1e-11), (MG_FP32, 1e-4)):
+        with CompositeSystem(topology, mg_cycle=cycle, mg_precision=precision) as s:
+            for seed in (1, 2):
+                r = np.where(active, np.random.default_rng(seed).standard_normal(n), 0.0)
+                want = oracle.precondition(r)
+                assert np.abs(s.precondition(r) - want)[active].max() <= bound * np.abs(want[active]).max(), (precision, seed)
+    oracle.close()
+    built.close()
+
+
 @pytest.mark.parametrize("cycle", [MG_CYCLE_REFERENCE, MG_CYCLE_COMPOSITE])
 def test_fine_level_of_a_large_grid(gpu, cycle):
     """More than 4,096 bricks: the two pre-sweeps as two launches, deferred rows of both levels; the
