@@ -249,8 +249,6 @@ namespace pcfd
             if (cycle == PCFD_MG_CYCLE_CORRECTED) { s.mg_prolong_scale = 2.0; s.mg_lattice_scale = 1.5; }
             if (cycle == PCFD_MG_CYCLE_COMPOSITE) s.mg_prolong_scale = 2.0;
             build_multigrid(s, t, diag);
-            for (MgLevel<double>& level : s.mg64) level.prolong = s.mg_lattice_scale;
-            for (MgLevel<float>& level : s.mg32) level.prolong = s.mg_lattice_scale;
             if (!options || !options->disable_fused_smoother) build_fine_smoother(s, t, diag);
             if (cycle == PCFD_MG_CYCLE_COMPOSITE)
             {

@@ -398,12 +398,21 @@ namespace pcfd
         levels.push_back(std::move(current));
         s.mg64.clear();
         s.mg32.clear();
+        // all of a level is set before the small ones are planned as one launch, which copies from them
         s.mg64.resize(levels.size());
-        for (size_t l = 0; l < levels.size(); ++l) upload_level(s.mg64[l], levels[l]);
+        for (size_t l = 0; l < levels.size(); ++l)
+        {
+            upload_level(s.mg64[l], levels[l]);
+            s.mg64[l].prolong = s.mg_lattice_scale;
+        }
         if (s.mg_precision == PCFD_MG_FP32)
         {
             s.mg32.resize(levels.size());
-            for (size_t l = 0; l < levels.size(); ++l) upload_level(s.mg32[l], levels[l]);
+            for (size_t l = 0; l < levels.size(); ++l)
+            {
+                upload_level(s.mg32[l], levels[l]);
+                s.mg32[l].prolong = s.mg_lattice_scale;
+            }
             plan_tail(s.mg32, host_rows(levels), kCoarsestSweeps, kOmega, s.mg_tail32);
         }
         plan_tail(s.mg64, host_rows(levels), kCoarsestSweeps, kOmega, s.mg_tail64);

@@ -84,6 +84,27 @@ def test_solves_with_finer_levels_outside_the_launch(gpu, cycle, precision):
 
 
 STAGE_SMOOTH = 2                      # PCFD_PROFILE_STAGE_SMOOTH
+MG_CYCLE_CORRECTED = 1
+
+
+@pytest.mark.parametrize("precision,bound", [(MG_FP64, 1e-12), (MG_FP32, 1e-4)])
+@pytest.mark.parametrize("cycle", [MG_CYCLE_REFERENCE, MG_CYCLE_CORRECTED, MG_CYCLE_COMPOSITE])
+def test_cycles_match_their_separate_launches(gpu, cycle, precision, bound):
+    """Every cycle against itself in launches of its own, each level with its own weights (the lattice
+    corrections of the corrected cycle count 1.5 times): bounds as for the oracle."""
+    built = grid(*GRIDS["ragged"])
+    act = built.active.astype(bool)
+    r = np.where(act, np.random.default_rng(6).standard_normal(built.storage_size), 0.0)
+    with CompositeSystem(built.topology, mg_cycle=cycle, mg_precision=precision) as s:
+        start = s.launch_count()
+        together = s.precondition(r)
+        middle = s.launch_count()
+        s.profile_begin(STAGE_SMOOTH, 64)
+        apart = s.precondition(r)
+        s.profile_end(64)
+        assert s.launch_count() - middle > middle - start + 4       # the levels did run apart
+    assert rel(together, apart, act) <= bound
+    built.close()
 
 
 @pytest.mark.parametrize("fp16", [0, 1])
