@@ -42,7 +42,9 @@ namespace pcfd
         if (!ok) throw Error(PCFD_INVALID_ARG, what);
     }
 
-    // Owning device buffer.
+    // Owning device buffer.  Its copies and clears run on the null stream, which the systems' own streams do
+    // not wait for, and neither ends with the host call (a copy returns once its source is staged): so
+    // each waits here before it returns.
     template <class T> struct DBuf
     {
         T* p = nullptr;
@@ -71,13 +73,18 @@ namespace pcfd
             cuda_check(cudaMalloc(&fresh, count * sizeof(T)), "cudaMalloc");
             p = static_cast<T*>(fresh);
             n = count;               // only now: callers test n for "is there"
-            if (zero) cuda_check(cudaMemset(p, 0, count * sizeof(T)), "cudaMemset");
+            if (!zero) return;
+            cuda_check(cudaMemset(p, 0, count * sizeof(T)), "cudaMemset");
+            complete();
         }
         void upload(const std::vector<T>& host)
         {
             alloc(host.size(), false);
-            if (!host.empty()) cuda_check(cudaMemcpy(p, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
+            if (host.empty()) return;
+            cuda_check(cudaMemcpy(p, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
+            complete();
         }
+        static void complete() { cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "null stream"); }
         operator T*() const { return p; }
     };
 

@@ -74,8 +74,21 @@ extern "C"
         return cudaSuccess;
     }
     cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
-    cudaError_t cudaMemset(void* p, int value, size_t bytes) { std::memset(p, value, bytes); return cudaSuccess; }
-    cudaError_t cudaMemcpy(void* to, const void* from, size_t bytes, cudaMemcpyKind) { std::memcpy(to, from, bytes); return cudaSuccess; }
+    // on the null stream, and done when something waits for it: a copy out of ordinary memory returns once
+    // the source has been staged, a memset at once
+    cudaError_t cudaMemset(void* p, int value, size_t bytes)
+    {
+        const Call call;
+        legacy[current].pending.push_back([=] { std::memset(p, value, bytes); });
+        return cudaSuccess;
+    }
+    cudaError_t cudaMemcpy(void* to, const void* from, size_t bytes, cudaMemcpyKind)
+    {
+        const Call call;
+        const std::vector<char> staged(static_cast<const char*>(from), static_cast<const char*>(from) + bytes);
+        legacy[current].pending.push_back([=] { std::memcpy(to, staged.data(), bytes); });
+        return cudaSuccess;
+    }
     cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) { *p = std::malloc(bytes); return cudaSuccess; }
     cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
     cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { a->type = cudaMemoryTypeUnregistered; return cudaSuccess; }
@@ -205,6 +218,16 @@ int main(int argc, char** argv)
             bool ok = download(s, 0, stream, 0, 1);
             for (int limit = 0; limit < 12 && ok; ++limit) ok = download(s, 0, stream, 0, 2 + limit, limit);
             return ok ? 0 : 1;
+        }
+        if (check == "uploads complete")
+        {
+            // what a stream that does not wait for the null stream would read right after the call
+            pcfd::DBuf<int> buffer;
+            buffer.upload(std::vector<int>(1000, 7));
+            if (buffer.p[0] != 7 || buffer.p[999] != 7) { std::puts("upload not complete"); return 1; }
+            buffer.alloc(1000);
+            if (buffer.p[0] != 0 || buffer.p[999] != 0) { std::puts("clearing not complete"); return 1; }
+            return 0;
         }
         if (check == "failed allocation")
         {

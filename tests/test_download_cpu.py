@@ -26,6 +26,7 @@ def test_threaded_download(probe, check):
     assert run.returncode == 0, run.stdout + run.stderr
 
 
-def test_failed_allocation_leaves_no_size(probe):
-    run = subprocess.run([probe, "failed allocation"], capture_output=True, text=True, timeout=60)
+@pytest.mark.parametrize("check", ["failed allocation", "uploads complete"])
+def test_device_buffers(probe, check):
+    run = subprocess.run([probe, check], capture_output=True, text=True, timeout=60)
     assert run.returncode == 0, run.stdout + run.stderr
